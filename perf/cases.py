@@ -8,6 +8,7 @@ bench.py's workloads.  Sizes run from one 2048 x 2048 projection of one row to a
     run(state)          one pass through the public entry points; returns its outputs
     work(case)          bytes and operations the pass cannot do without
     tolerance(case)     how far another correct implementation may be off
+    exact(case, seed)   the outputs of run() as plain 64-bit arithmetic gives them
 """
 import numpy as np
 import torch
@@ -104,10 +105,9 @@ def _lengths(batch, longest):
     return [longest - (i * longest) // (2 * batch) for i in range(batch)]
 
 
-def _engine(case, g, max_seq, batch, rows):
+def _weights(case, g):
+    """The model's weights one after another: (embedding, final norm, head), then a dict per layer."""
     layers, H, Nq, Nkv, I = SHAPES[case["model"]]
-    engine = Qwen3Engine(EngineConfig(n_layers=layers, hidden=H, n_q_heads=Nq, n_kv_heads=Nkv, head_dim=HEAD, inter=I, vocab=VOCAB,
-                                      group=GROUP, max_seq=max_seq, max_batch=batch, max_rows=rows, act_mode=2))
 
     def norm(n):
         return (1.0 + _normal(g, n, std=0.02)).bfloat16()
@@ -116,14 +116,23 @@ def _engine(case, g, max_seq, batch, rows):
     # peaked: the head of token t points along the embedding of token t - 1, so greedy decoding has a clear winner.
     out_std = 0.02 / (2 * layers) ** 0.5
     embed = _normal(g, VOCAB, H, std=0.5).bfloat16()
-    head = (torch.roll(embed, 1, 0) * 0.04).contiguous()
-    engine.load_globals(embed, norm(H), head)
-    del embed, head
-    for i in range(layers):
+    yield embed, norm(H), (torch.roll(embed, 1, 0) * 0.04).contiguous()
+    del embed
+    for _ in range(layers):
         w = {"input_norm": norm(H), "post_norm": norm(H), "q_norm": norm(HEAD), "k_norm": norm(HEAD)}
         for name, K, N, std in (("qkv", H, (Nq + 2 * Nkv) * HEAD, 0.02), ("o", Nq * HEAD, H, out_std), ("gu", H, 2 * I, 0.02),
                                 ("down", I, H, out_std)):
             w[name + "_qw"], w[name + "_qz"], w[name + "_s"] = _quantised(g, K, N, std)
+        yield w
+
+
+def _engine(case, g, max_seq, batch, rows):
+    layers, H, Nq, Nkv, I = SHAPES[case["model"]]
+    engine = Qwen3Engine(EngineConfig(n_layers=layers, hidden=H, n_q_heads=Nq, n_kv_heads=Nkv, head_dim=HEAD, inter=I, vocab=VOCAB,
+                                      group=GROUP, max_seq=max_seq, max_batch=batch, max_rows=rows, act_mode=2))
+    weights = _weights(case, g)
+    engine.load_globals(*next(weights))
+    for i, w in enumerate(weights):
         engine.load_layer(i, w)
     return engine
 
@@ -239,3 +248,86 @@ def tolerance(case):
     # all layers: 1.2e-3; 6.3e-3 of the logits against projections with un-rounded fp32 activations, and as much between
     # two passes over the same inputs, because reductions arrive in another order.  The tokens agreed throughout.
     return {"rel": 5e-3, "max": 2.5e-2, "differ": 0.01}
+
+
+# ---- the same in 64 bits ------------------------------------------------------------------------------------------------
+def _dense(qweight, qzeros, scales):
+    """The matrix of an INT4-AWQ triple: column c of a word lies in nibble c / 2 (even c) or 4 + c / 2 (odd c)."""
+    shifts = torch.tensor([4 * (c // 2 + 4 * (c % 2)) for c in range(8)], device="cuda", dtype=torch.int32)
+    q, z = (((w.unsqueeze(-1) >> shifts) & 15).flatten(1).to(torch.int8) for w in (qweight, qzeros))
+    K, N = q.shape
+    return ((q.view(-1, GROUP, N) - z.unsqueeze(1)).double() * scales.double().unsqueeze(1)).view(K, N)
+
+
+def _attend(q, k, v, start):
+    """Causal attention of the rows at positions start, start + 1, ...: q [n, heads, HEAD], k and v [positions, kv heads, HEAD]"""
+    n, heads, _ = q.shape
+    k, v = (t.repeat_interleave(heads // t.shape[1], 1).transpose(0, 1) for t in (k, v))
+    score = q.transpose(0, 1) @ k.transpose(1, 2) / HEAD ** 0.5
+    late = torch.arange(k.shape[1], device="cuda") > start + torch.arange(n, device="cuda").unsqueeze(1)
+    return (score.masked_fill_(late, float("-inf")).softmax(-1) @ v).transpose(0, 1)
+
+
+def _norm64(x, w):
+    return x / (x.square().mean(-1, keepdim=True) + 1e-6).sqrt() * w.double()
+
+
+def _rotate(x, pos):
+    angle = pos.double().unsqueeze(1) * 1e6 ** (-torch.arange(0, HEAD, 2, device="cuda").double() / HEAD)
+    c, s = angle.cos().unsqueeze(1), angle.sin().unsqueeze(1)
+    a, b = x[..., :HEAD // 2], x[..., HEAD // 2:]
+    return torch.cat((a * c - b * s, b * c + a * s), -1)
+
+
+class _Model64:
+    def __init__(self, case, g):
+        _, _, self.Nq, self.Nkv, self.I = SHAPES[case["model"]]
+        weights = _weights(case, g)
+        self.embed, self.norm, self.head = next(weights)
+        self.layers = list(weights)
+        self.cache = [{} for _ in self.layers]
+
+    def forward(self, runs):
+        """runs: (slot, first position, tokens) per sequence; logits of the last token of each."""
+        def product(x, name):
+            return x @ _dense(w[name + "_qw"], w[name + "_qz"], w[name + "_s"])
+
+        ids = torch.from_numpy(np.concatenate([np.asarray(t, np.int64) for _, _, t in runs])).cuda()
+        pos = torch.cat([p + torch.arange(len(t), device="cuda") for _, p, t in runs])
+        sizes = [len(t) for _, _, t in runs]
+        h = self.embed[ids].double()
+        for w, cache in zip(self.layers, self.cache):
+            q, k, v = product(_norm64(h, w["input_norm"]), "qkv").view(len(ids), -1, HEAD).split((self.Nq, self.Nkv, self.Nkv), 1)
+            q, k = _rotate(_norm64(q, w["q_norm"]), pos), _rotate(_norm64(k, w["k_norm"]), pos)
+            out = []
+            for (slot, p, _), qs, ks, vs in zip(runs, q.split(sizes), k.split(sizes), v.split(sizes)):
+                if p:
+                    ks, vs = torch.cat((cache[slot][0], ks)), torch.cat((cache[slot][1], vs))
+                cache[slot] = (ks, vs)
+                out.append(_attend(qs, ks, vs, p))
+            h = h + product(torch.cat(out).flatten(1), "o")
+            gate, up = product(_norm64(h, w["post_norm"]), "gu").split(self.I, 1)
+            h = h + product(torch.nn.functional.silu(gate) * up, "down")
+        last = h[torch.tensor(sizes, device="cuda").cumsum(0) - 1]
+        return _norm64(last, self.norm) @ self.head.double().T
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    if kind in ("proj", "attn"):
+        state = prepare(case, seed)
+        if kind == "proj":
+            return state["x"].double() @ _dense(*state["w"])
+        return torch.stack([_attend(state["q"][b:b + 1].double(), k[:, :n].double().transpose(0, 1), v[:, :n].double().transpose(0, 1), n)[0]
+                            for b, (k, v, n) in enumerate(zip(state["k"], state["v"], state["len"].tolist()))])
+    g, ids = _generator(seed), np.random.default_rng(seed)
+    model = _Model64(case, g)
+    if kind == "prefill":
+        prompts, steps = [ids.integers(0, VOCAB, case["prompt"])], 1
+    else:
+        prompts, steps = [ids.integers(0, VOCAB, m) for m in _lengths(case["batch"], case["prompt"])], DECODE_STEPS
+    logits = model.forward([(b, 0, p) for b, p in enumerate(prompts)])
+    for s in range(steps):
+        token = logits.argmax(1).tolist()
+        logits = model.forward([(b, len(p) + s, [t]) for b, (p, t) in enumerate(zip(prompts, token))])
+    return {"tokens": None, "logits": logits}
