@@ -596,14 +596,40 @@ __global__ void __launch_bounds__(kGemmThreads3, 2) awq_gemm_tc3_kernel(const Ge
     }
 }
 
+// Calls of few rows read the weights through the packed-word kernel of awq_gemm_rows.cu.  Up to 32 rows that is one pass and
+// always ahead of the 128-row tiles (4096 x 24576: 8 rows 14.7 against 45.9 us, 16 rows 17.2, 32 rows 33.0 against 46.4).
+// More rows repeat the pass, which pays while the passes together read at most about 4000 units of 16 KB (64 rows:
+// 2560 x 19456 31.6 against 33.8 us, 4096 x 24576 54.9 against 48.6; 96 rows: 9728 x 2560 23.5 against 48.9 us,
+// 2560 x 19456 42.3 against 38.2).
+int g_gemm_rows_max = 96;  // tuning key "gemm_rows_max": most rows of such a call; 0 switches the path off
+bool rows_pay(int M, int K, int N) {
+    return M <= 32 || (long long)((M + 31) / 32) * ((N + 255) / 256) * (K / 128) <= 4000;
+}
+
 constexpr int kMaxSplitK = 8;
 int g_gemm_split_k = 1;  // tuning key "gemm_split_k": 0 switches the K split of the third generation off
 int g_gemm_impl = 3;  // 3: mbarrier hand-over to a dedicated MMA warp (default); 2: stages handed over at a block-wide barrier (tuning key "gemm_impl")
 
 }  // namespace
 
+int awq_rows_launch(const __half* x16, const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales, float* y, const float* residual,
+                    int M, int K, int N, cudaStream_t stream);
+int awq_rows_status();
+void awq_rows_set_tuning(const char* key, int value);
+
+// x (n4 float4s) -> fp16; also zeroes zero4 float4s
+int convert_f16_launch(const float* x, __half* out, int64_t n4, float* zero, int64_t zero4, cudaStream_t stream) {
+    int blocks = int(((n4 > zero4 ? n4 : zero4) + 255) / 256);
+    if (blocks > 148 * 8) blocks = 148 * 8;
+    return pdl_status(launch_pdl(convert_f16_kernel, dim3(blocks), dim3(256), 0, stream, reinterpret_cast<const float4*>(x),
+                                 reinterpret_cast<uint2*>(out), n4, reinterpret_cast<float4*>(zero), zero4),
+                      "awq_gemm convert");
+}
+
 void awq_gemm_set_tuning(const char* key, int value) {
     if (!strcmp(key, "gemm_impl")) g_gemm_impl = value == 3 ? 3 : 2;
+    if (!strcmp(key, "gemm_rows_max")) g_gemm_rows_max = value < 0 ? 0 : value;
+    awq_rows_set_tuning(key, value);
     if (!strcmp(key, "gemm_split_k")) g_gemm_split_k = value < 0 ? 0 : value;
 }
 
@@ -614,6 +640,7 @@ using namespace kuiper;
 extern "C" int kuiper_awq_gemm_status(void) {
     int v = 0;
     if (cudaMemcpyFromSymbol(&v, g_gemm_wait_error, sizeof(int)) != cudaSuccess) v = -1;
+    if (v == 0) v = awq_rows_status();
     if (v == 0) return KUIPER_OK;
     set_error("awq_gemm: a bounded tensor-core pipeline wait ran out (code %d)", v);
     return KUIPER_INTERNAL_ERROR;
@@ -649,6 +676,18 @@ static int gemm_common(const float* x, const __half* x16_in, const int32_t* qwei
                                          (reinterpret_cast<uintptr_t>(workspace) & 15) == 0),
                    "awq_gemm: needs a 16-byte aligned workspace of kuiper_awq_gemm_workspace_bytes(M, K) bytes (got %zu)",
                    workspace_bytes);
+    const int64_t n4 = x16_in ? 0 : int64_t(M) * K / 4;  // activations that arrive as fp16 need no conversion
+    __half* const x16_ws = reinterpret_cast<__half*>(workspace);
+    const bool few_rows = g_gemm_impl == 3 && g_gemm_split_k == 1 && M <= g_gemm_rows_max && rows_pay(M, K, N) && N % 32 == 0 &&
+                          ((reinterpret_cast<uintptr_t>(qweight) | reinterpret_cast<uintptr_t>(qzeros)) & 15) == 0;
+    if (few_rows) {
+        const int64_t zero4 = p.mode != 2 ? int64_t(M) * N / 4 : 0;
+        if (n4 > 0 || zero4 > 0) {
+            const int rc = convert_f16_launch(x, x16_ws, n4, y, zero4, as_stream(stream));
+            if (rc != KUIPER_OK) return rc;
+        }
+        return awq_rows_launch(x16_in ? x16_in : x16_ws, qweight, qzeros, scales, y, p.mode == 1 ? residual : nullptr, M, K, N, as_stream(stream));
+    }
     // Few output tiles (a decode batch, a short chunk: one row of tiles is N / 256 CTAs) leave most SMs without work while
     // every CTA streams a whole column panel of the weight: the third generation then splits K so that about two CTAs
     // per SM are busy.  A split is a whole number of 128-row groups; the sums meet through reductions, so y starts from
@@ -664,20 +703,14 @@ static int gemm_common(const float* x, const __half* x16_in, const int32_t* qwei
     }
     const bool zero_y = splits > 1 && p.mode != 2;
     // activations converted to fp16 once (the same launch zeroes y for a split call), then 128 x 256 output tiles
-    const int64_t n4 = x16_in ? 0 : int64_t(M) * K / 4;  // activations that arrive as fp16 need no conversion
     const int64_t zero4 = zero_y ? int64_t(M) * N / 4 : 0;
     if (n4 > 0 || zero4 > 0) {
-        int blocks = int(((n4 > zero4 ? n4 : zero4) + 255) / 256);
-        if (blocks > 148 * 8) blocks = 148 * 8;
-        int rc = pdl_status(launch_pdl(convert_f16_kernel, dim3(blocks), dim3(256), 0, as_stream(stream),
-                                       reinterpret_cast<const float4*>(x), reinterpret_cast<uint2*>(workspace), n4,
-                                       reinterpret_cast<float4*>(y), zero4),
-                            "awq_gemm convert");
+        const int rc = convert_f16_launch(x, x16_ws, n4, y, zero4, as_stream(stream));
         if (rc != KUIPER_OK) return rc;
     }
     GemmParams2 p2;
     p2.g = p;
-    p2.x16 = x16_in ? x16_in : reinterpret_cast<const __half*>(workspace);
+    p2.x16 = x16_in ? x16_in : x16_ws;
     p2.tiles_per_split = 0;
     const size_t smem2 = 1024 + size_t(kStages2) * (kStageA2 + kStageB2);
     if (g_gemm_impl == 3) {

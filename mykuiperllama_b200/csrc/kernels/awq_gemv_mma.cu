@@ -1168,6 +1168,9 @@ int awq_gemv_trace_read(long long* out, int max_values) {
 }
 #endif
 
+// the same map for the kernels that read a weight matrix in other units (boxes of 32 words x 32 rows, 128-byte swizzle)
+bool awq_weight_map(const int32_t* qweight, int K, int N, CUtensorMap* out) { return get_map_mma(qweight, K, N, out); }
+
 void awq_gemv_mma_set_tuning(const char* key, int value) {
     if (!strcmp(key, "gemv_dyn_pct")) g_dyn_pct = value < 0 ? 0 : value;
     if (!strcmp(key, "gemv_dyn_chunk")) g_dyn_chunk = value < 0 ? 0 : value;

@@ -40,9 +40,11 @@ public:
     // where RMSNorm(input) / SwiGLU(input) is written when the row count takes the tensor-core path, which has
     // no fused prologue ([max rows, dim1] fp32)
     void set_norm_scratch(const tensor::Tensor& scratch) { norm_scratch_ = scratch; }
-    // quantised layers, fp16-operand mode: inputs of at least this many rows go to the tcgen05 GEMM instead of
-    // the GEMV (0 = never).  With its K split (few output tiles -> several CTAs per tile) the GEMM is ahead of passes of
-    // 4 rows through the GEMV from 16 rows on (4096 x 24576, 16 rows: 48 us against 4 x 12.8 us; 32 rows: 48.5 against 102).
+    // quantised layers, fp16-operand mode: inputs of at least this many rows go to the GEMM entry (packed-word kernel up to
+    // about a hundred rows, tcgen05 tiles beyond) instead of the GEMV in passes of four rows (0 = never).  One pass of the
+    // GEMV also runs the input norm / SwiGLU itself, which saves four launches a layer: Qwen3-8B decode of two sequences
+    // takes the same time either way (1.82 ms a step, 0.6B 0.71 against 0.82), of three 1.97 against 2.13, of five
+    // 2.00 against 3.35.
     void set_gemm_min_rows(int32_t rows) { gemm_min_rows_ = rows; }
     // scratch of the split-K kernel: kernel::matmul_quant_workspace_bytes(M, K, N) bytes, zero-initialised once
     void set_workspace(const tensor::Tensor& workspace);
@@ -75,7 +77,7 @@ private:
     tensor::Tensor gemm_workspace_;
     tensor::Tensor norm_scratch_;
     tensor::Tensor tickets_;
-    int32_t gemm_min_rows_ = 16;  // from 16 rows on the split-K tcgen05 GEMM beats passes of 4 rows through the GEMV
+    int32_t gemm_min_rows_ = 3;
 };
 }  // namespace op
 
