@@ -20,6 +20,7 @@
 //
 // Every mbarrier wait is bounded; on a timeout the CTA records an error word, stops issuing work,
 // still frees its tensor memory and returns.
+#include <cuda.h>
 #include <cstring>
 
 #include "common.cuh"
@@ -596,15 +597,402 @@ __global__ void __launch_bounds__(kGemmThreads3, 2) awq_gemm_tc3_kernel(const Ge
     }
 }
 
-// Calls of few rows read the weights through the packed-word kernel of awq_gemm_rows.cu.  Up to 32 rows that is one pass and
-// always ahead of the 128-row tiles (4096 x 24576: 8 rows 14.7 against 45.9 us, 16 rows 17.2, 32 rows 33.0 against 46.4).
-// More rows repeat the pass, which pays while the passes together read at most about 4000 units of 16 KB (64 rows:
-// 2560 x 19456 31.6 against 33.8 us, 4096 x 24576 54.9 against 48.6; 96 rows: 9728 x 2560 23.5 against 48.9 us,
-// 2560 x 19456 42.3 against 38.2).
-int g_gemm_rows_max = 96;  // tuning key "gemm_rows_max": most rows of such a call; 0 switches the path off
-bool rows_pay(int M, int K, int N) {
-    return M <= 32 || (long long)((M + 31) / 32) * ((N + 255) / 256) * (K / 128) <= 4000;
+// ---------------------------------------------------------------------------------------------
+// Calls of many rows: 256 x 256 output tiles, so that every dequantised weight feeds two 128-row MMAs.
+// The 128-row kernel above is bound by the issue of the dequantisation (342 warp instructions per warp and 64-row stage
+// against 512 tensor-pipe cycles); with 256 rows the same instructions stand against 1024 cycles, and the activations
+// come by TMA instead of cp.async.  One CTA per SM: 512 TMEM columns (two 128 x 256 accumulators), three stages of 64 KB
+// (2 x 16 KB activations, 32 KB weights).  Warps 0-15 dequantise and write results, warp 16 issues the MMAs, warp 17 the
+// activation boxes.  The dequantising warps form two halves that fill alternate stages: with eight warps a stage took
+// 1900 cycles, most of them waiting (for packed words, for the stage, for stores to become visible).  The weight tile is
+// MN-major, so that a packed word becomes one 16-byte store without a transposition and a warp reads its words in
+// 128-byte runs.
+// Work is dealt in units of one quantisation group (128 weight rows) of one tile: every CTA takes an equal run of the
+// units of the full-height tiles and an equal run of those of the last, shorter tile row, so there is no partial wave
+// whatever the shape.  Results leave through a 2 KB shared-memory patch per warp and TMA: a plain store where the run
+// covered the whole contraction and y is to be overwritten, else an fp32 add-reduction.
+constexpr int kTileM4 = 256, kTileN4 = 256, kStages4 = 3;
+constexpr int kStageA4 = kTileM4 * kBK * 2, kStageB4 = kTileN4 * kBK * 2;  // 32 KB each
+constexpr int kBlockB4 = kBK * 128;  // 64 weight rows of 64 columns
+constexpr int kPatch4 = 32 * 16 * 4;
+constexpr int kHalfThreads4 = 256;                // the warps that fill one stage; two such halves take turns
+constexpr int kThreads4 = 2 * kHalfThreads4 + 64;
+constexpr size_t kSmem4 = 1024 + size_t(kStages4) * (kStageA4 + kStageB4) + 16 * kPatch4;
+
+struct GemmCall4 {
+    CUtensorMap x_map;      // fp16 activations [M, K], box 64 x 128 rows, 128-byte swizzle
+    CUtensorMap y_map;      // y [M, N], box 16 columns x 32 rows, 64-byte swizzle
+    const uint32_t* qw;
+    const uint32_t* qz;
+    const __half* scales;
+    const float* residual;  // rides with the first group of a tile
+    int M, K, N;
+    int add;                // 1: y already holds the addend (or zeros): every result is added
+    int m_tiles, n_tiles, groups;
+    int full_units, full_run;  // units of the tile rows of 256 rows; units of them per CTA
+    int tail_units, tail_run;  // the same for a last tile row of fewer rows
+};
+
+__global__ void __launch_bounds__(kThreads4, 1) awq_gemm_tc4_kernel(const __grid_constant__ GemmCall4 p) {
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t smem = (smem_addr(smem_raw) + 1023u) & ~1023u;
+    const uint32_t sA = smem, sB = smem + kStages4 * kStageA4, sY = sB + kStages4 * kStageB4;
+    __shared__ uint64_t full_bar[kStages4], free_bar[kStages4], tile_bar, drained_bar;
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_dead;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+    if (tid == 0) {
+#pragma unroll
+        for (int i = 0; i < kStages4; i++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&full_bar[i])), "r"(uint32_t(kHalfThreads4 / 32 + 1)));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&free_bar[i])));
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&drained_bar)), "r"(uint32_t(2 * kHalfThreads4 / 32)));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&tile_bar)));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        s_dead = 0;
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    pdl_launch_dependents();
+
+    // ---- this CTA's units: a run of the full tile rows, then a run of the last tile row.  Unit u of a segment with T tile
+    // rows is group u % groups of tile u / groups, whose row index runs fastest (neighbouring CTAs share weights)
+    const int full_rows = p.m_tiles - (p.tail_units > 0 ? 1 : 0);
+    const int f0 = min(int(blockIdx.x) * p.full_run, p.full_units), f1 = min(f0 + p.full_run, p.full_units);
+    // the tail is dealt from the last CTA down: it evens out the run that the last CTAs have less of
+    const int rb = int(gridDim.x) - 1 - int(blockIdx.x);
+    const int t0 = min(rb * p.tail_run, p.tail_units), t1 = min(t0 + p.tail_run, p.tail_units);
+    const int n_units = (f1 - f0) + (t1 - t0);
+    struct Unit { int mt, nt, group; };
+    auto unit_at = [&](int i) {
+        Unit r;
+        int u = f0 + i;
+        if (u < f1) {
+            const int tile = u / p.groups;
+            r.group = u - tile * p.groups;
+            r.nt = tile / full_rows;
+            r.mt = tile - r.nt * full_rows;
+        } else {
+            u = t0 + (i - (f1 - f0));
+            r.nt = u / p.groups;
+            r.group = u - r.nt * p.groups;
+            r.mt = full_rows;
+        }
+        return r;
+    };
+    auto unit_after = [&](int i, const Unit& u) {  // unit i + 1, where unit i is u
+        if (u.group + 1 == p.groups || f0 + i + 1 == f1) return unit_at(i + 1);
+        return Unit{u.mt, u.nt, u.group + 1};
+    };
+    // the run leaves a tile after unit i
+    auto tile_ends = [&](int i, int group) { return group + 1 == p.groups || i + 1 == n_units || f0 + i + 1 == f1; };
+
+    if (warp == 17) {
+        // ------------------------------------------------------------ activations
+        if (lane == 0) {
+            pdl_wait();
+            bool dead = false;
+            int it = 0;
+            Unit u = {0, 0, 0};
+            for (int i = 0; i < n_units && !dead; i++) {
+                u = i == 0 ? unit_at(0) : unit_after(i - 1, u);
+                const int boxes = p.M - u.mt * kTileM4 > kBM ? 2 : 1;
+                for (int h = 0; h < 2; h++, it++) {
+                    const int s = it % kStages4;
+                    if (it >= kStages4 && !tc_mbar_wait(&free_bar[s], uint32_t(it / kStages4 - 1) & 1u)) {
+                        atomicExch(&g_gemm_wait_error, 21);
+                        s_dead = 1;
+                        dead = true;
+                        break;
+                    }
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&full_bar[s])),
+                                 "r"(uint32_t(boxes * kStageA2))
+                                 : "memory");
+                    for (int b = 0; b < boxes; b++)
+                        asm volatile(
+                            "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                            ::"r"(sA + s * kStageA4 + b * kStageA2), "l"(&p.x_map), "r"(u.group * 128 + h * kBK),
+                            "r"(u.mt * kTileM4 + b * kBM), "r"(smem_addr(&full_bar[s]))
+                            : "memory");
+                }
+            }
+            // after a failed wait the copies in flight still have to land before the block may end
+            if (dead)
+                for (int j = it - kStages4 < 0 ? 0 : it - kStages4; j < it; j++) tc_mbar_wait(&full_bar[j % kStages4], uint32_t(j / kStages4) & 1u);
+        }
+    } else if (warp == 16) {
+        // ------------------------------------------------------------ MMA issue
+        if (lane == 0) {
+            const uint32_t idesc = (1u << 4) | (1u << 16) | (uint32_t(kTileN4 >> 3) << 17) | (uint32_t(kBM >> 4) << 24);  // B is MN-major
+            bool dead = false, fresh = true;  // fresh: the next MMA starts a tile
+            int it = 0, tiles = 0;
+            Unit u = {0, 0, 0};
+            for (int i = 0; i < n_units && !dead; i++) {
+                u = i == 0 ? unit_at(0) : unit_after(i - 1, u);
+                const int halves = p.M - u.mt * kTileM4 > kBM ? 2 : 1;
+                // a new tile overwrites the accumulators: every warp has to have read the last one's
+                if (fresh && tiles > 0 && !tc_mbar_wait(&drained_bar, uint32_t(tiles - 1) & 1u)) {
+                    atomicExch(&g_gemm_wait_error, 25);
+                    s_dead = 1;
+                    break;
+                }
+                for (int h = 0; h < 2; h++, it++) {
+                    const int s = it % kStages4;
+                    if (!tc_mbar_wait(&full_bar[s], uint32_t(it / kStages4) & 1u)) {
+                        atomicExch(&g_gemm_wait_error, 22);
+                        s_dead = 1;
+                        dead = true;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    for (int m = 0; m < halves; m++) {
+#pragma unroll
+                        for (int kk = 0; kk < kBK / 16; kk++) {
+                            const uint64_t adesc = make_desc(sA + s * kStageA4 + m * kStageA2 + kk * 32);
+                            const uint64_t bdesc = make_desc(sB + s * kStageB4 + kk * 2048) | (uint64_t(kBlockB4 >> 4) << 16);
+                            const uint32_t accumulate = (fresh && kk == 0) ? 0u : 1u;
+                            asm volatile(
+                                "{\n\t.reg .pred p;\n\t"
+                                "setp.ne.b32 p, %4, 0;\n\t"
+                                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                                ::"r"(tmem + m * kTileN4), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+                                : "memory");
+                        }
+                    }
+                    fresh = false;
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(&free_bar[s]))
+                                 : "memory");
+                }
+                if (tile_ends(i, u.group)) {
+                    fresh = true;
+                    tiles++;
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(&tile_bar))
+                                 : "memory");
+                }
+            }
+        }
+    } else {
+        // ------------------------------------------------------------ dequantisation and results
+        const int NW = p.N >> 3;
+        const int half = warp >> 3;                                // fills the stages 2 i + half
+        const int koct = warp & 7, j = lane;  // eight weight rows of packed word column j: a warp reads 128-byte runs
+        auto load_w = [&](const Unit& u, uint32_t (&w)[8]) {
+            const int wcol = u.nt * (kTileN4 / 8) + j;
+            const bool ok = wcol < NW;
+            const uint32_t* src = p.qw + size_t(u.group * 128 + half * kBK + koct * 8) * NW + (ok ? wcol : 0);
+#pragma unroll
+            for (int r = 0; r < 8; r++) w[r] = ok ? __ldg(src + size_t(r) * NW) : 0u;
+        };
+        auto load_consts = [&](const Unit& u, uint32_t& zw, uint4& sraw) {
+            const int wcol = u.nt * (kTileN4 / 8) + j;
+            const bool ok = wcol < NW;
+            zw = ok ? __ldg(p.qz + size_t(u.group) * NW + wcol) : 0u;
+            sraw = ok ? __ldg(reinterpret_cast<const uint4*>(p.scales + size_t(u.group) * p.N) + wcol) : make_uint4(0, 0, 0, 0);
+        };
+        // a word's eight columns are a 16-byte chunk of its row: column block j / 8, chunk (j % 8) ^ (row % 8)
+        uint32_t b_off[8];
+#pragma unroll
+        for (int r = 0; r < 8; r++) b_off[r] = uint32_t((j >> 3) * kBlockB4 + (koct * 8 + r) * 128 + (((j & 7) ^ r) << 4));
+        bool dead = false;
+        TileConsts tc;
+        auto stage_step = [&](int it, const uint32_t (&w)[8]) {
+            const int s = it % kStages4;
+            if (it >= kStages4 && !dead && !tc_mbar_wait(&free_bar[s], uint32_t(it / kStages4 - 1) & 1u)) {
+                atomicExch(&g_gemm_wait_error, 23);
+                s_dead = 1;
+                dead = true;
+            }
+            const uint32_t dst = sB + s * kStageB4;
+#pragma unroll
+            for (int r = 0; r < 8; r++) {
+                uint32_t d[4];
+                dequant_word_consts(w[r], tc, d);
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + b_off[r]), "r"(d[0]), "r"(d[1]), "r"(d[2]), "r"(d[3]) : "memory");
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&full_bar[s])) : "memory");
+        };
+
+        uint32_t w[8], zw = 0;
+        uint4 sraw = make_uint4(0, 0, 0, 0);
+        Unit next = {0, 0, 0};
+        if (n_units > 0) {
+            next = unit_at(0);
+            load_w(next, w);
+            load_consts(next, zw, sraw);
+        }
+        int first_group = next.group;  // group at which the run entered the current tile
+        bool waited = false;
+        int tiles = 0;
+        for (int i = 0; i < n_units; i++) {
+            const Unit u = next;
+            const bool more = i + 1 < n_units;
+            if (more) next = unit_after(i, u);
+            tc = make_tile_consts(zw, sraw);
+            if (more) load_consts(next, zw, sraw);
+            stage_step(2 * i + half, w);
+            if (more) load_w(next, w);
+            if (!tile_ends(i, u.group)) continue;
+
+            // ---- results: every MMA of the tile is done (a barrier of its own: a half sees only every other phase of free_bar)
+            if (!dead && !tc_mbar_wait(&tile_bar, uint32_t(tiles++) & 1u)) {
+                atomicExch(&g_gemm_wait_error, 24);
+                s_dead = 1;
+                dead = true;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (!waited) {
+                pdl_wait();  // y (and the residual) belong to the preceding kernels until here
+                waited = true;
+            }
+            const bool whole = first_group == 0 && u.group + 1 == p.groups;
+            const bool add = p.add || !whole;
+            // two accumulators: one per half; one accumulator: each half takes half of the columns
+            const bool both = p.M - u.mt * kTileM4 > kBM;
+            const int m = both ? half : 0, chunks = both ? 8 : 4, c0 = both ? 0 : half * 4;
+            if (!dead) {
+#pragma unroll 1
+                for (int c = 0; c < chunks; c++) {
+                    const int row0 = u.mt * kTileM4 + m * kBM + (warp & 3) * 32;
+                    const int tcol = ((warp >> 2) & 1) * 128 + (c0 + c) * 16, col0 = u.nt * kTileN4 + tcol;
+                    if (row0 >= p.M || col0 >= p.N) break;
+                    uint32_t r[16];
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                        : "r"(tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(m * kTileN4 + tcol))
+                        : "memory");
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (p.residual && first_group == 0 && row0 + lane < p.M) {
+                        const float* rp = p.residual + size_t(row0 + lane) * p.N + col0;
+#pragma unroll
+                        for (int v = 0; v < 4; v++)
+                            if (col0 + v * 4 < p.N) {
+                                const float4 a = __ldcg(reinterpret_cast<const float4*>(rp) + v);
+                                r[4 * v] = __float_as_uint(__uint_as_float(r[4 * v]) + a.x);
+                                r[4 * v + 1] = __float_as_uint(__uint_as_float(r[4 * v + 1]) + a.y);
+                                r[4 * v + 2] = __float_as_uint(__uint_as_float(r[4 * v + 2]) + a.z);
+                                r[4 * v + 3] = __float_as_uint(__uint_as_float(r[4 * v + 3]) + a.w);
+                            }
+                    }
+                    // three patches in turn: the warp's own, and its share of the stage that its half fills next (no MMA
+                    // reads a stage now); a patch is free once the box sent from it has been read
+                    const uint32_t patch = c % 3 == 0 ? sY + warp * kPatch4
+                                                      : sB + ((2 * i + 2 + half) % kStages4) * kStageB4 + ((warp & 7) * 2 + c % 3 - 1) * kPatch4;
+                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 2;" ::: "memory");
+                    __syncwarp();
+#pragma unroll
+                    for (int v = 0; v < 4; v++)
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(patch + lane * 64 + ((v ^ ((lane >> 1) & 3)) << 4)), "r"(r[4 * v]),
+                                     "r"(r[4 * v + 1]), "r"(r[4 * v + 2]), "r"(r[4 * v + 3])
+                                     : "memory");
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (add)
+                            asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%1, %2}], [%3];" ::"l"(&p.y_map),
+                                         "r"(col0), "r"(row0), "r"(patch)
+                                         : "memory");
+                        else
+                            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(&p.y_map), "r"(col0),
+                                         "r"(row0), "r"(patch)
+                                         : "memory");
+                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    }
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + half), "n"(kHalfThreads4) : "memory");  // the stage is the half's again
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&drained_bar)) : "memory");
+            first_group = more ? next.group : 0;
+        }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
+
+using EncodeTiledTc = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledTc encode_fn_tc() {
+    static EncodeTiledTc fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) f = nullptr;
+        return reinterpret_cast<EncodeTiledTc>(f);
+    }();
+    return fn;
+}
+// row-major [rows, cols], boxes of box_cols (box_cols * elem_bytes = the swizzle's span) x box_rows, zero fill
+bool encode_rows_map(CUtensorMap* out, CUtensorMapDataType type, int elem_bytes, const void* base, int rows, int cols, int box_cols, int box_rows,
+                     CUtensorMapSwizzle swizzle) {
+    EncodeTiledTc fn = encode_fn_tc();
+    if (!fn) return false;
+    const cuuint64_t dims[2] = {cuuint64_t(cols), cuuint64_t(rows)};
+    const cuuint64_t strides[1] = {cuuint64_t(cols) * elem_bytes};
+    const cuuint32_t box[2] = {cuuint32_t(box_cols), cuuint32_t(box_rows)};
+    const cuuint32_t estr[2] = {1, 1};
+    return fn(out, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+int g_gemm_tile_rows = 33;  // tuning key "gemm_tile_rows": fewest rows of a call that takes the 256 x 256 tiles; 0: none
+
+// The 256 x 256 tiles lead everywhere (4096 x 24576: 64 rows 39.7 against 48.6 us, 256 rows 54 / 88, 512 rows 97 / 163, 2048
+// rows 362 / 703) but for one case: between 257 and 511 rows they run a second, short tile row with its own unpacking and
+// results, and the 128-row kernel is ahead where its K split happens to fill one wave of two CTAs per SM (4096 x 6144, 300
+// rows: 34.0 against 38.1 us, 4096 x 2560 23.4 / 28.6; where it does not: 2560 x 6144 39.1 / 24.6).
+bool tiles_pay(int M, int tiles128, int splits128) {
+    const int ctas = tiles128 * splits128, sms = device_sm_count();
+    return M <= 256 || M >= 512 || ctas * 2 < sms * 3 || ctas > 2 * sms;
+}
+
+// y[add ? += : =] x16 . W (+ residual); unless add, y has been zeroed
+int launch_tiles4(const GemmParams& g, const __half* x16, cudaStream_t stream) {
+    GemmCall4 c;
+    memset(&c, 0, sizeof(c));
+    if (!encode_rows_map(&c.x_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x16, g.M, g.K, kBK, kBM, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !encode_rows_map(&c.y_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, g.y, g.M, g.N, 16, 32, CU_TENSOR_MAP_SWIZZLE_64B)) {
+        set_error("awq_gemm: tensor map encoding failed");
+        return KUIPER_INTERNAL_ERROR;
+    }
+    c.qw = g.qw; c.qz = g.qz; c.scales = g.scales;
+    c.residual = g.mode == 1 ? g.residual : nullptr;
+    c.M = g.M; c.K = g.K; c.N = g.N;
+    c.add = g.mode == 2;
+    c.m_tiles = (g.M + kTileM4 - 1) / kTileM4;
+    c.n_tiles = (g.N + kTileN4 - 1) / kTileN4;
+    c.groups = g.K / 128;
+    const int tail = g.M % kTileM4 != 0 ? 1 : 0, ctas = device_sm_count();
+    c.full_units = (c.m_tiles - tail) * c.n_tiles * c.groups;
+    c.tail_units = tail * c.n_tiles * c.groups;
+    c.full_run = (c.full_units + ctas - 1) / ctas;
+    c.tail_run = (c.tail_units + ctas - 1) / ctas;
+    static size_t configured[kMaxDevices] = {};
+    if (!ensure_dynamic_smem(awq_gemm_tc4_kernel, kSmem4, configured)) {
+        set_error("awq_gemm: cannot reserve %zu bytes of shared memory", kSmem4);
+        return KUIPER_INTERNAL_ERROR;
+    }
+    return pdl_status(launch_pdl(awq_gemm_tc4_kernel, dim3(ctas), dim3(kThreads4), kSmem4, stream, c), "awq_gemm");
+}
+
+// Calls of up to 32 rows read the weights through the packed-word kernel of awq_gemm_rows.cu, one pass over them: 4096 x 24576
+// 8 rows 14.7, 16 rows 17.2, 32 rows 33.0 us, where the 256 x 256 tiles take 39 us from one row to 64 (they are bound by
+// the dequantisation there) and the 128-row tiles 46.
+int g_gemm_rows_max = 32;  // tuning key "gemm_rows_max": most rows of such a call; 0 switches the path off
 
 constexpr int kMaxSplitK = 8;
 int g_gemm_split_k = 1;  // tuning key "gemm_split_k": 0 switches the K split of the third generation off
@@ -628,6 +1016,7 @@ int convert_f16_launch(const float* x, __half* out, int64_t n4, float* zero, int
 
 void awq_gemm_set_tuning(const char* key, int value) {
     if (!strcmp(key, "gemm_impl")) g_gemm_impl = value == 3 ? 3 : 2;
+    if (!strcmp(key, "gemm_tile_rows")) g_gemm_tile_rows = value < 0 ? 0 : value;
     if (!strcmp(key, "gemm_rows_max")) g_gemm_rows_max = value < 0 ? 0 : value;
     awq_rows_set_tuning(key, value);
     if (!strcmp(key, "gemm_split_k")) g_gemm_split_k = value < 0 ? 0 : value;
@@ -678,7 +1067,7 @@ static int gemm_common(const float* x, const __half* x16_in, const int32_t* qwei
                    workspace_bytes);
     const int64_t n4 = x16_in ? 0 : int64_t(M) * K / 4;  // activations that arrive as fp16 need no conversion
     __half* const x16_ws = reinterpret_cast<__half*>(workspace);
-    const bool few_rows = g_gemm_impl == 3 && g_gemm_split_k == 1 && M <= g_gemm_rows_max && rows_pay(M, K, N) && N % 32 == 0 &&
+    const bool few_rows = g_gemm_impl == 3 && g_gemm_split_k == 1 && M <= g_gemm_rows_max && N % 32 == 0 &&
                           ((reinterpret_cast<uintptr_t>(qweight) | reinterpret_cast<uintptr_t>(qzeros)) & 15) == 0;
     if (few_rows) {
         const int64_t zero4 = p.mode != 2 ? int64_t(M) * N / 4 : 0;
@@ -700,6 +1089,15 @@ static int gemm_common(const float* x, const __half* x16_in, const int32_t* qwei
         for (int sdiv = 2; sdiv <= groups && sdiv <= kMaxSplitK && sdiv <= want; sdiv++)
             if (groups % sdiv == 0) splits = sdiv;
         if (g_gemm_split_k > 1 && groups % g_gemm_split_k == 0) splits = g_gemm_split_k;  // forced (measurement aid)
+    }
+    if (g_gemm_impl == 3 && g_gemm_split_k == 1 && g_gemm_tile_rows > 0 && M >= g_gemm_tile_rows && encode_fn_tc() != nullptr &&
+        tiles_pay(M, int(grid2.x * grid2.y), splits)) {
+        const int64_t zero4 = p.mode != 2 ? int64_t(M) * N / 4 : 0;
+        if (n4 > 0 || zero4 > 0) {
+            const int rc = convert_f16_launch(x, x16_ws, n4, y, zero4, as_stream(stream));
+            if (rc != KUIPER_OK) return rc;
+        }
+        return launch_tiles4(p, x16_in ? x16_in : x16_ws, as_stream(stream));
     }
     const bool zero_y = splits > 1 && p.mode != 2;
     // activations converted to fp16 once (the same launch zeroes y for a split call), then 128 x 256 output tiles
