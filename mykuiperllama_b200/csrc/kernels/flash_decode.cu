@@ -1191,6 +1191,9 @@ size_t flash_slots(int M) {
 
 }  // namespace
 
+void flash_prefill_set_tuning(const char* key, int value);
+int flash_prefill_tc_status();
+
 void flash_decode_set_tuning(const char* key, int value) {
     if (!strcmp(key, "flash_splits")) g_force_splits = value;
     if (!strcmp(key, "flash_drop_slice")) g_flash_drop_slice = value;
@@ -1199,6 +1202,7 @@ void flash_decode_set_tuning(const char* key, int value) {
     if (!strcmp(key, "flash_mma")) g_flash_mma = value;
     if (!strcmp(key, "flash_mma_fused")) g_flash_mma_fused = value;
     if (!strcmp(key, "flash_wide")) g_flash_wide = value;
+    flash_prefill_set_tuning(key, value);
 }
 
 }  // namespace kuiper
@@ -1221,6 +1225,10 @@ extern "C" int kuiper_flash_decode_status(void) {
     int v = 0;
     const int zero = 0;
     if (cudaMemcpyFromSymbol(&v, g_flash_wait_error, sizeof(int)) != cudaSuccess) v = -1;
+    if (v == 0 && flash_prefill_tc_status() != 0) {
+        set_error("flash_prefill: a bounded tensor-core pipeline wait ran out (code %d)", flash_prefill_tc_status());
+        return KUIPER_INTERNAL_ERROR;
+    }
     if (v == 0) return KUIPER_OK;
     cudaMemcpyToSymbol(g_flash_wait_error, &zero, sizeof(int));  // reported once
     set_error("flash_decode: the combining CTA's bounded wait for the other slices ran out (code %d)", v);

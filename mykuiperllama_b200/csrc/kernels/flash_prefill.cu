@@ -259,7 +259,20 @@ int launch_prefill(const PrefillParams& p, cudaStream_t stream) {
     return pdl_status(launch_pdl(kern, grid, dim3(kPWarps * 32), smem, stream, p), "flash_prefill");
 }
 
+// The tcgen05 kernel takes calls of at least this many (row, head) vectors per kv head, or of 256 rows (tuning key
+// "prefill_tc_vectors", 0: none).  32 / 8 heads: 128 rows 11.2 us there against 9.9 here, 256 rows 14.6 / 18.6, 512 rows
+// 21.9 / 36.3, 2048 rows 101 / 305, 2048 rows behind 2048 217 / 793; 16 / 8 heads: 77 rows 10.6 / 9.2, 256 rows 14.5 / 15.5.
+int g_prefill_tc_vectors = 1024;
+
 }  // namespace
+
+bool flash_prefill_tc_launch(const float* q, const uint16_t* kcache, const uint16_t* vcache, float* out, int M, int Nq, int Nkv, int max_seq,
+                             int n_slots, int pos0, int slot, cudaStream_t stream, int* rc);
+
+void flash_prefill_set_tuning(const char* key, int value) {
+    if (!strcmp(key, "prefill_tc_vectors")) g_prefill_tc_vectors = value < 0 ? 0 : value;
+}
+
 }  // namespace kuiper
 
 using namespace kuiper;
@@ -278,6 +291,10 @@ extern "C" int kuiper_flash_prefill(const float* q, const uint16_t* kcache, cons
     KUIPER_REQUIRE(Nkv <= 65535, "flash_prefill: grid too large");
     const int R = Nq / Nkv;
     KUIPER_REQUIRE(R == 1 || R == 2 || R == 4 || R == 8, "flash_prefill: group size %d is not supported", R);
+    int rc = KUIPER_OK;
+    if (g_prefill_tc_vectors > 0 && (M * R >= g_prefill_tc_vectors || M >= 256) &&
+        flash_prefill_tc_launch(q, kcache, vcache, out, M, Nq, Nkv, max_seq, n_slots, pos0, slot, as_stream(stream), &rc))
+        return rc;
     PrefillParams p;
     p.q = q; p.kc = kcache; p.vc = vcache; p.out = out;
     p.M = M; p.Nq = Nq; p.Nkv = Nkv; p.max_seq = max_seq; p.pos0 = pos0; p.slot = slot;
