@@ -607,9 +607,9 @@ __global__ void __launch_bounds__(kGemmThreads3, 2) awq_gemm_tc3_kernel(const Ge
 // 1900 cycles, most of them waiting (for packed words, for the stage, for stores to become visible).  The weight tile is
 // MN-major, so that a packed word becomes one 16-byte store without a transposition and a warp reads its words in
 // 128-byte runs.
-// Work is dealt in units of one quantisation group (128 weight rows) of one tile: every CTA takes an equal run of the
-// units of the full-height tiles and an equal run of those of the last, shorter tile row, so there is no partial wave
-// whatever the shape.  Results leave through a 2 KB shared-memory patch per warp and TMA: a plain store where the run
+// Every CTA takes as many whole tiles as all CTAs can have.  What is left is dealt in units of one quantisation group (128
+// weight rows) of one tile: an equal run of the units of the remaining full-height tiles and an equal run of those of the
+// last, shorter tile row, so there is no partial wave whatever the shape.  Results leave through a 2 KB shared-memory patch per warp and TMA: a plain store where the run
 // covered the whole contraction and y is to be overwritten, else an fp32 add-reduction.
 constexpr int kTileM4 = 256, kTileN4 = 256, kStages4 = 3;
 constexpr int kStageA4 = kTileM4 * kBK * 2, kStageB4 = kTileN4 * kBK * 2;  // 32 KB each
@@ -629,7 +629,8 @@ struct GemmCall4 {
     int M, K, N;
     int add;                // 1: y already holds the addend (or zeros): every result is added
     int m_tiles, n_tiles, groups;
-    int full_units, full_run;  // units of the tile rows of 256 rows; units of them per CTA
+    int whole_tiles;           // tiles that a CTA has to itself; they come first
+    int full_units, full_run;  // end of the units of the tile rows of 256 rows; units of them per CTA behind the whole tiles
     int tail_units, tail_run;  // the same for a last tile row of fewer rows
 };
 
@@ -663,25 +664,26 @@ __global__ void __launch_bounds__(kThreads4, 1) awq_gemm_tc4_kernel(const __grid
     const uint32_t tmem = s_tmem;
     pdl_launch_dependents();
 
-    // ---- this CTA's units: a run of the full tile rows, then a run of the last tile row.  Unit u of a segment with T tile
+    // ---- this CTA's units: whole tiles, a run of the other full tile rows, a run of the last tile row.  Unit u of the full
     // rows is group u % groups of tile u / groups, whose row index runs fastest (neighbouring CTAs share weights)
     const int full_rows = p.m_tiles - (p.tail_units > 0 ? 1 : 0);
-    const int f0 = min(int(blockIdx.x) * p.full_run, p.full_units), f1 = min(f0 + p.full_run, p.full_units);
+    const int n_whole = p.whole_tiles * p.groups, w0 = int(blockIdx.x) * n_whole;
+    const int f0 = min(int(gridDim.x) * n_whole + int(blockIdx.x) * p.full_run, p.full_units), f1 = min(f0 + p.full_run, p.full_units);
+    const int n_full = n_whole + f1 - f0;
     // the tail is dealt from the last CTA down: it evens out the run that the last CTAs have less of
     const int rb = int(gridDim.x) - 1 - int(blockIdx.x);
     const int t0 = min(rb * p.tail_run, p.tail_units), t1 = min(t0 + p.tail_run, p.tail_units);
-    const int n_units = (f1 - f0) + (t1 - t0);
+    const int n_units = n_full + t1 - t0;
     struct Unit { int mt, nt, group; };
     auto unit_at = [&](int i) {
         Unit r;
-        int u = f0 + i;
-        if (u < f1) {
-            const int tile = u / p.groups;
+        if (i < n_full) {
+            const int u = i < n_whole ? w0 + i : f0 + i - n_whole, tile = u / p.groups;
             r.group = u - tile * p.groups;
             r.nt = tile / full_rows;
             r.mt = tile - r.nt * full_rows;
         } else {
-            u = t0 + (i - (f1 - f0));
+            const int u = t0 + i - n_full;
             r.nt = u / p.groups;
             r.group = u - r.nt * p.groups;
             r.mt = full_rows;
@@ -689,11 +691,11 @@ __global__ void __launch_bounds__(kThreads4, 1) awq_gemm_tc4_kernel(const __grid
         return r;
     };
     auto unit_after = [&](int i, const Unit& u) {  // unit i + 1, where unit i is u
-        if (u.group + 1 == p.groups || f0 + i + 1 == f1) return unit_at(i + 1);
+        if (u.group + 1 == p.groups || i + 1 == n_full) return unit_at(i + 1);
         return Unit{u.mt, u.nt, u.group + 1};
     };
     // the run leaves a tile after unit i
-    auto tile_ends = [&](int i, int group) { return group + 1 == p.groups || i + 1 == n_units || f0 + i + 1 == f1; };
+    auto tile_ends = [&](int i, int group) { return group + 1 == p.groups || i + 1 == n_units || i + 1 == n_full; };
 
     if (warp == 17) {
         // ------------------------------------------------------------ activations
@@ -960,7 +962,15 @@ bool tiles_pay(int M, int tiles128, int splits128) {
     return M <= 256 || M >= 512 || ctas * 2 < sms * 3 || ctas > 2 * sms;
 }
 
-// y[add ? += : =] x16 . W (+ residual); unless add, y has been zeroed
+// zeroes what a launch that overwrites y adds up from several CTAs: columns [col0, N) of every row and the rows from row0 on
+__global__ void __launch_bounds__(256) zero_split_kernel(float4* y, int M, int N4, int row0, int col4) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int m = blockIdx.x;
+    for (int i = (m >= row0 ? 0 : col4) + threadIdx.x; i < N4; i += 256) y[size_t(m) * N4 + i] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// y[add ? += : =] x16 . W (+ residual)
 int launch_tiles4(const GemmParams& g, const __half* x16, cudaStream_t stream) {
     GemmCall4 c;
     memset(&c, 0, sizeof(c));
@@ -979,12 +989,22 @@ int launch_tiles4(const GemmParams& g, const __half* x16, cudaStream_t stream) {
     const int tail = g.M % kTileM4 != 0 ? 1 : 0, ctas = device_sm_count();
     c.full_units = (c.m_tiles - tail) * c.n_tiles * c.groups;
     c.tail_units = tail * c.n_tiles * c.groups;
-    c.full_run = (c.full_units + ctas - 1) / ctas;
+    c.whole_tiles = (c.m_tiles - tail) * c.n_tiles / ctas;
+    const int split_units = c.full_units - c.whole_tiles * ctas * c.groups;
+    c.full_run = (split_units + ctas - 1) / ctas;
     c.tail_run = (c.tail_units + ctas - 1) / ctas;
     static size_t configured[kMaxDevices] = {};
     if (!ensure_dynamic_smem(awq_gemm_tc4_kernel, kSmem4, configured)) {
         set_error("awq_gemm: cannot reserve %zu bytes of shared memory", kSmem4);
         return KUIPER_INTERNAL_ERROR;
+    }
+    if (!c.add && (split_units > 0 || tail)) {
+        const int full_rows = c.m_tiles - tail;
+        const int first_col = split_units > 0 ? c.whole_tiles * ctas / full_rows * kTileN4 : g.N;  // the first column tile that is not whole
+        const int rc = pdl_status(launch_pdl(zero_split_kernel, dim3(g.M), dim3(256), 0, stream, reinterpret_cast<float4*>(g.y), g.M, g.N / 4,
+                                             full_rows * kTileM4, first_col / 4),
+                                  "awq_gemm zero");
+        if (rc != KUIPER_OK) return rc;
     }
     return pdl_status(launch_pdl(awq_gemm_tc4_kernel, dim3(ctas), dim3(kThreads4), kSmem4, stream, c), "awq_gemm");
 }
@@ -1092,9 +1112,8 @@ static int gemm_common(const float* x, const __half* x16_in, const int32_t* qwei
     }
     if (g_gemm_impl == 3 && g_gemm_split_k == 1 && g_gemm_tile_rows > 0 && M >= g_gemm_tile_rows && encode_fn_tc() != nullptr &&
         tiles_pay(M, int(grid2.x * grid2.y), splits)) {
-        const int64_t zero4 = p.mode != 2 ? int64_t(M) * N / 4 : 0;
-        if (n4 > 0 || zero4 > 0) {
-            const int rc = convert_f16_launch(x, x16_ws, n4, y, zero4, as_stream(stream));
+        if (n4 > 0) {
+            const int rc = convert_f16_launch(x, x16_ws, n4, nullptr, 0, as_stream(stream));
             if (rc != KUIPER_OK) return rc;
         }
         return launch_tiles4(p, x16_in ? x16_in : x16_ws, as_stream(stream));

@@ -48,16 +48,20 @@ __global__ void add_kernel(const float* __restrict__ a, const float* __restrict_
 }
 
 // ---------------------------------------------------------------- rmsnorm
-// One CTA of 1024 threads per token row.  The row is read once, with every load of a thread issued
-// before the first use (a single CTA is latency bound, so rounds of dependent loads are what costs).
+// One CTA per token row.  The row is read once, with every load of a thread issued before the first use (a single CTA is
+// latency bound, so rounds of dependent loads are what costs).  A few rows take 1024 threads each, for the shortest chain; a
+// prompt chunk takes 256 threads each, so that an SM works on eight rows at a time and not on two (2048 rows of 4096: 26 us
+// with 1024 threads).
 constexpr int kNormThreads = 1024;
-constexpr int kNormVec = 4;  // float4 per thread held in registers: rows up to 16384 wide
+constexpr int kNormThreadsChunk = 256;
+constexpr int kNormVec = 4;  // float4 per thread held in registers: rows up to 16384 (4096) wide
 
-__device__ __forceinline__ float block_sum_1024(float v, float* s_part) {
+template <int THREADS>
+__device__ __forceinline__ float block_sum(float v, float* s_part) {
     v = warp_sum(v);
     if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = v;
     __syncthreads();
-    float tot = (threadIdx.x & 31) < (kNormThreads / 32) ? s_part[threadIdx.x & 31] : 0.f;
+    float tot = (threadIdx.x & 31) < (THREADS / 32) ? s_part[threadIdx.x & 31] : 0.f;
     return warp_sum(tot);  // every warp reduces the 32 partials itself: same order, same value everywhere
 }
 
@@ -71,23 +75,23 @@ __device__ __forceinline__ void norm_store4(__half* y, int i4, float4 o) {
     reinterpret_cast<uint2*>(y)[i4] = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
 
-template <typename OUT>
-__global__ void __launch_bounds__(kNormThreads) rmsnorm_kernel(const float* x, const uint16_t* __restrict__ w, OUT* y, int H,
+template <typename OUT, int THREADS>
+__global__ void __launch_bounds__(THREADS) rmsnorm_kernel(const float* x, const uint16_t* __restrict__ w, OUT* y, int H,
                                                                float eps) {
-    __shared__ float s_part[kNormThreads / 32];
+    __shared__ float s_part[THREADS / 32];
     pdl_launch_dependents();
     pdl_wait();
     const float* xr = x + size_t(blockIdx.x) * H;
     OUT* yr = y + size_t(blockIdx.x) * H;
     const int t = threadIdx.x;
-    if ((H & 3) == 0 && H <= kNormThreads * kNormVec * 4 && (reinterpret_cast<uintptr_t>(xr) & 15) == 0 &&
+    if ((H & 3) == 0 && H <= THREADS * kNormVec * 4 && (reinterpret_cast<uintptr_t>(xr) & 15) == 0 &&
         (reinterpret_cast<uintptr_t>(yr) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 7) == 0) {
         const int n4 = H >> 2;
         float4 v[kNormVec];
         uint2 wv[kNormVec];
 #pragma unroll
         for (int j = 0; j < kNormVec; j++) {
-            const int i = t + j * kNormThreads;
+            const int i = t + j * THREADS;
             v[j] = i < n4 ? __ldcg(reinterpret_cast<const float4*>(xr) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
             wv[j] = i < n4 ? __ldg(reinterpret_cast<const uint2*>(w) + i) : make_uint2(0, 0);
         }
@@ -97,10 +101,10 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_kernel(const float* x, c
             ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss);
             ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
         }
-        const float rstd = 1.0f / sqrtf(block_sum_1024(ss, s_part) / float(H) + eps);
+        const float rstd = 1.0f / sqrtf(block_sum<THREADS>(ss, s_part) / float(H) + eps);
 #pragma unroll
         for (int j = 0; j < kNormVec; j++) {
-            const int i = t + j * kNormThreads;
+            const int i = t + j * THREADS;
             if (i < n4) {
                 float4 o;
                 o.x = (v[j].x * rstd) * bf16_lo(wv[j].x); o.y = (v[j].y * rstd) * bf16_hi(wv[j].x);
@@ -112,15 +116,36 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_kernel(const float* x, c
     }
     // any width / alignment: two scalar passes
     float ss = 0.f;
-    for (int i = t; i < H; i += kNormThreads) {
+    for (int i = t; i < H; i += THREADS) {
         const float a = xr[i];
         ss = fmaf(a, a, ss);
     }
-    const float rstd = 1.0f / sqrtf(block_sum_1024(ss, s_part) / float(H) + eps);
-    for (int i = t; i < H; i += kNormThreads) norm_store(yr, i, (xr[i] * rstd) * bf16_bits_to_float(w[i]));
+    const float rstd = 1.0f / sqrtf(block_sum<THREADS>(ss, s_part) / float(H) + eps);
+    for (int i = t; i < H; i += THREADS) norm_store(yr, i, (xr[i] * rstd) * bf16_bits_to_float(w[i]));
 }
 
 // ---------------------------------------------------------------- swiglu
+// A prompt chunk is bound by memory (2048 rows of 2 x 12288: 251 MB read and written), so four elements per access where
+// the rows allow it; element by element otherwise.
+__device__ __forceinline__ float swiglu_value(float g, float u) { return (g / (1.0f + expf(-g))) * u; }
+
+template <typename OUT>
+__global__ void __launch_bounds__(256) swiglu4_kernel(float* gate_up, OUT* out, int M, int I4, int clear_input) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int64_t total = int64_t(M) * I4;
+    float4* gu = reinterpret_cast<float4*>(gate_up);
+    for (int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < total; idx += int64_t(gridDim.x) * blockDim.x) {
+        const int64_t m = idx / I4, at = m * I4 + idx;  // row m of gate: m * 2 * I4 + (idx - m * I4)
+        const float4 g = __ldcg(gu + at), u = __ldcg(gu + at + I4);
+        norm_store4(out + 4 * m * I4, int(idx - m * I4), make_float4(swiglu_value(g.x, u.x), swiglu_value(g.y, u.y), swiglu_value(g.z, u.z), swiglu_value(g.w, u.w)));
+        if (clear_input) {
+            gu[at] = make_float4(0.f, 0.f, 0.f, 0.f);
+            gu[at + I4] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+}
+
 template <typename OUT>
 __global__ void swiglu_kernel(float* gate_up, OUT* out, int M, int I, int clear_input) {
     pdl_launch_dependents();
@@ -129,7 +154,7 @@ __global__ void swiglu_kernel(float* gate_up, OUT* out, int M, int I, int clear_
     for (int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < total; idx += int64_t(gridDim.x) * blockDim.x) {
         const int64_t m = idx / I, i = idx - m * I;
         const float g = gate_up[m * 2 * I + i], u = gate_up[m * 2 * I + I + i];
-        norm_store(out + idx, 0, (g / (1.0f + expf(-g))) * u);
+        norm_store(out + idx, 0, swiglu_value(g, u));
         if (clear_input) {  // leave the projection buffer zeroed for the next accumulating matmul
             gate_up[m * 2 * I + i] = 0.f;
             gate_up[m * 2 * I + I + i] = 0.f;
@@ -281,6 +306,22 @@ int grid_for(int64_t work_items, int threads) {
     return int(blocks < 1 ? 1 : (blocks > cap ? cap : blocks));
 }
 
+template <typename OUT>
+int launch_rmsnorm(const float* x, const uint16_t* w, OUT* y, int M, int H, float eps, cudaStream_t stream, const char* what) {
+    if (M >= 2 * device_sm_count() && H <= kNormThreadsChunk * kNormVec * 4)
+        return pdl_status(launch_pdl(rmsnorm_kernel<OUT, kNormThreadsChunk>, dim3(M), dim3(kNormThreadsChunk), 0, stream, x, w, y, H, eps), what);
+    return pdl_status(launch_pdl(rmsnorm_kernel<OUT, kNormThreads>, dim3(M), dim3(kNormThreads), 0, stream, x, w, y, H, eps), what);
+}
+
+template <typename OUT>
+int launch_swiglu(float* gate_up, OUT* out, int M, int I, int clear_input, cudaStream_t stream, const char* what) {
+    if (I % 4 == 0 && ((reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0)
+        return pdl_status(launch_pdl(swiglu4_kernel<OUT>, dim3(grid_for(int64_t(M) * I / 4, 256)), dim3(256), 0, stream, gate_up, out, M, I / 4,
+                                     clear_input), what);
+    return pdl_status(launch_pdl(swiglu_kernel<OUT>, dim3(grid_for(int64_t(M) * I, 256)), dim3(256), 0, stream, gate_up, out, M, I, clear_input),
+                      what);
+}
+
 }  // namespace
 }  // namespace kuiper
 
@@ -322,29 +363,26 @@ extern "C" int kuiper_rmsnorm_f32(const float* x, const uint16_t* w, float* y, i
                                   kuiper_stream_t stream) {
     KUIPER_REQUIRE(x && w && y, "rmsnorm: null tensor pointer");
     KUIPER_REQUIRE(M > 0 && H > 0, "rmsnorm: empty shape M=%d H=%d", M, H);
-    return pdl_status(launch_pdl(rmsnorm_kernel<float>, dim3(M), dim3(kNormThreads), 0, as_stream(stream), x, w, y, H, eps), "rmsnorm");
+    return launch_rmsnorm(x, w, y, M, H, eps, as_stream(stream), "rmsnorm");
 }
 
 extern "C" int kuiper_rmsnorm_f16(const float* x, const uint16_t* w, uint16_t* y16, int M, int H, float eps,
                                   kuiper_stream_t stream) {
     KUIPER_REQUIRE(x && w && y16, "rmsnorm_f16: null tensor pointer");
     KUIPER_REQUIRE(M > 0 && H > 0, "rmsnorm_f16: empty shape M=%d H=%d", M, H);
-    return pdl_status(launch_pdl(rmsnorm_kernel<__half>, dim3(M), dim3(kNormThreads), 0, as_stream(stream), x, w,
-                                 reinterpret_cast<__half*>(y16), H, eps), "rmsnorm_f16");
+    return launch_rmsnorm(x, w, reinterpret_cast<__half*>(y16), M, H, eps, as_stream(stream), "rmsnorm_f16");
 }
 
 extern "C" int kuiper_swiglu_f32(float* gate_up, float* out, int M, int I, int clear_input, kuiper_stream_t stream) {
     KUIPER_REQUIRE(gate_up && out, "swiglu: null tensor pointer");
     KUIPER_REQUIRE(M > 0 && I > 0, "swiglu: empty shape M=%d I=%d", M, I);
-    return pdl_status(launch_pdl(swiglu_kernel<float>, dim3(grid_for(int64_t(M) * I, 256)), dim3(256), 0, as_stream(stream), gate_up, out, M, I,
-                                 clear_input), "swiglu");
+    return launch_swiglu(gate_up, out, M, I, clear_input, as_stream(stream), "swiglu");
 }
 
 extern "C" int kuiper_swiglu_f16(float* gate_up, uint16_t* out16, int M, int I, int clear_input, kuiper_stream_t stream) {
     KUIPER_REQUIRE(gate_up && out16, "swiglu_f16: null tensor pointer");
     KUIPER_REQUIRE(M > 0 && I > 0, "swiglu_f16: empty shape M=%d I=%d", M, I);
-    return pdl_status(launch_pdl(swiglu_kernel<__half>, dim3(grid_for(int64_t(M) * I, 256)), dim3(256), 0, as_stream(stream), gate_up,
-                                 reinterpret_cast<__half*>(out16), M, I, clear_input), "swiglu_f16");
+    return launch_swiglu(gate_up, reinterpret_cast<__half*>(out16), M, I, clear_input, as_stream(stream), "swiglu_f16");
 }
 
 extern "C" int kuiper_embedding_bf16(const int32_t* tokens, const uint16_t* table, float* out, int M, int H,

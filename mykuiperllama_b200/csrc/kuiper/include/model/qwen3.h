@@ -119,6 +119,9 @@ private:
     bool rows_are_chunk_ = false;
     int32_t chunk_pos0_ = 0, chunk_slot_ = 0;
     static constexpr int32_t kPrefillAttentionMinRows = 16;
+    // from here on the GEMM's tiles are mostly whole ones that it stores without adding (fewer rows: every tile is shared by
+    // several CTAs, and zeroing it in the rotary kernel costs nothing extra)
+    static constexpr int32_t kOverwriteRows = 512;
 };
 
 }  // namespace model

@@ -46,6 +46,13 @@ public:
     // takes the same time either way (1.82 ms a step, 0.6B 0.71 against 0.82), of three 1.97 against 2.13, of five
     // 2.00 against 3.35.
     void set_gemm_min_rows(int32_t rows) { gemm_min_rows_ = rows; }
+    // accumulate mode: passes of at least this many rows overwrite the output instead (0 = never), so that nobody has to
+    // zero it; the engine sets it for the projections whose addend is zero.  Clearing gate|up before and reading it back for
+    // the addition cost a 2048-row chunk of the Qwen3-8B shape 150 us a layer.
+    void set_overwrite_rows(int32_t rows) { overwrite_rows_ = rows; }
+    bool overwrites(int32_t rows) const {
+        return is_quant_layer_ && act_mode_ != 0 && overwrite_rows_ > 0 && rows >= overwrite_rows_ && gemm_min_rows_ > 0 && rows >= gemm_min_rows_;
+    }
     // scratch of the split-K kernel: kernel::matmul_quant_workspace_bytes(M, K, N) bytes, zero-initialised once
     void set_workspace(const tensor::Tensor& workspace);
     // scratch of the tensor-core path: kernel::matmul_quant_gemm_workspace_bytes(max rows, dim1) bytes, no
@@ -78,6 +85,7 @@ private:
     tensor::Tensor norm_scratch_;
     tensor::Tensor tickets_;
     int32_t gemm_min_rows_ = 3;
+    int32_t overwrite_rows_ = 0;
 };
 }  // namespace op
 

@@ -30,6 +30,9 @@ public:
         clear_extra_row_ = row_elems;
     }
 
+    // off: the next pass leaves the qkv input and the extra buffer as they are (its projections overwrite them)
+    void set_clear_enabled(bool on) { clear_enabled_ = on; }
+
     // Decode batches only (one token row per sequence slot, seq_len == pos + 1): rotary, KV append and
     // flash-decoding in one kernel.  Inputs as for forward() plus seq_len; attention_out [M, Nq*D] replaces the q
     // output; workspace as for op::MultiHeadAttention; fresh_rows as documented there.
@@ -45,7 +48,7 @@ protected:
 private:
     int32_t head_num_ = 0, kv_head_num_ = 0, head_size_ = 0;
     float eps_ = 1e-6f;
-    bool clear_input_ = false;
+    bool clear_input_ = false, clear_enabled_ = true;
     tensor::Tensor key_cache_, value_cache_, clear_extra_, attention_workspace_;
     int32_t clear_extra_row_ = 0;
 };

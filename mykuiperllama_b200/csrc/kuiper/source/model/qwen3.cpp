@@ -225,6 +225,8 @@ base::Status Qwen3Model::init(base::DeviceType device_type) {
         L.down = make_quant(sh_down, c.tp_size == 1 && !accumulate_);
         for (op::MatmulLayer* m : {L.qkv.get(), L.gate_up.get()}) m->set_accumulate(accumulate_cols_);
         for (op::MatmulLayer* m : {L.o.get(), L.down.get()}) m->set_accumulate(accumulate_);
+        if (accumulate_ && accumulate_cols_)
+            for (op::MatmulLayer* m : {L.qkv.get(), L.gate_up.get()}) m->set_overwrite_rows(kOverwriteRows);
         if (accumulate_cols_) {
             // the two pre-norms run inside the projections that consume them
             L.qkv->set_input_norm(L.input_norm->get_weight(0), c.eps);
@@ -610,7 +612,10 @@ base::Status Qwen3Model::run_pass(int32_t M, bool inputs_settled) {
     };
 
     RETURN_IF_ERROR(embedding_->forward(tokens, h));
+    // a prompt chunk writes the projections' outputs anew in every layer; decode passes add into zeroed ones
+    const bool overwrite = !layers_.empty() && layers_[0].qkv->overwrites(M);
     for (Qwen3Layer& L : layers_) {
+        L.rope->set_clear_enabled(!overwrite);
         if (accumulate_cols_) {
             RETURN_IF_ERROR(L.qkv->forward(h, qkv));  // RMSNorm fused into the projection
         } else {
@@ -649,6 +654,10 @@ base::Status Qwen3Model::run_pass(int32_t M, bool inputs_settled) {
             RETURN_IF_ERROR(project_and_reduce(*L.down, act));
         }
     }
+    // the next pass that adds finds zeros again: it has fewer than kOverwriteRows rows (the rotary kernel of its first layer
+    // zeroes gate|up)
+    if (overwrite)
+        CUDA_OK(cudaMemsetAsync(const_cast<float*>(qkv.ptr<float>()), 0, size_t(kOverwriteRows) * QKV * sizeof(float), stream()));
     if (logit_rows_ > 0) {
         // logits only for the last logit_rows_ rows of the pass
         const int32_t r0 = M - logit_rows_;

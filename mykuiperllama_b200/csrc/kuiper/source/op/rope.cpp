@@ -60,7 +60,7 @@ base::Status RoPELayer::forward() {
     base::Status status = check();
     if (!status) return status;
     tensor::Tensor extra;
-    if (!clear_extra_.is_empty() && clear_extra_row_ > 0) {
+    if (clear_enabled_ && !clear_extra_.is_empty() && clear_extra_row_ > 0) {
         const int32_t row = (head_num_ + 2 * kv_head_num_) * head_size_;
         const int32_t M = int32_t(get_input(0).size() / size_t(row));
         if (size_t(M) * size_t(clear_extra_row_) > clear_extra_.size())
@@ -71,7 +71,7 @@ base::Status RoPELayer::forward() {
     }
     kernel::get_rope_kernel(device_type_)(get_input(0), get_weight(0), get_weight(1), get_input(3), get_input(4),
                                           get_input(1), get_input(2), get_output(0), key_cache_, value_cache_, head_num_,
-                                          kv_head_num_, head_size_, eps_, clear_input_,
+                                          kv_head_num_, head_size_, eps_, clear_input_ && clear_enabled_,
                                           extra.is_empty() ? nullptr : &extra, stream());
     return base::error::success();
 }
@@ -94,7 +94,7 @@ base::Status RoPELayer::forward_with_attention(const tensor::Tensor& qkv, const 
     if (status && seq_len.size() < size_t(M)) status = base::error::invalid_argument("seq_len tensor is too short.");
     if (!status) return status;
     tensor::Tensor extra;
-    if (!clear_extra_.is_empty() && clear_extra_row_ > 0) {
+    if (clear_enabled_ && !clear_extra_.is_empty() && clear_extra_row_ > 0) {
         if (size_t(M) * size_t(clear_extra_row_) > clear_extra_.size())
             return base::error::invalid_argument("the extra buffer is smaller than the pass");
         extra = tensor::Tensor(base::DataType::DataTypeFp32, std::vector<int32_t>{M, clear_extra_row_}, false, nullptr,
@@ -103,7 +103,7 @@ base::Status RoPELayer::forward_with_attention(const tensor::Tensor& qkv, const 
     }
     kernel::get_rope_mha_kernel(device_type_)(qkv, get_weight(0), get_weight(1), cos_cache, sin_cache, pos, seq_len, slot,
                                               attention_out, key_cache_, value_cache_, head_num_, kv_head_num_, head_size_,
-                                              eps_, fresh_rows, clear_input_, extra.is_empty() ? nullptr : &extra,
+                                              eps_, fresh_rows, clear_input_ && clear_enabled_, extra.is_empty() ? nullptr : &extra,
                                               attention_workspace_, stream());
     return base::error::success();
 }
