@@ -332,14 +332,19 @@ struct RowsPlan {
 };
 int g_rows_min_run = 1;  // tuning key "rows_min_run"
 
-RowsPlan plan_rows(int M, int K, int N) {
+RowsPlan plan_rows(int M, int K, int N, bool ordered) {
     RowsPlan r;
     r.nt = M <= 8 ? 1 : (M <= 16 ? 2 : 4);
     r.passes = (M + 8 * r.nt - 1) / (8 * r.nt);
-    r.occ = r.nt == 4 ? 2 : 3;
     r.tiles = (N + kTileCols - 1) / kTileCols;
     r.groups = K / kGroupRows;
     r.units = r.tiles * r.groups;
+    // Three CTAs per SM stream a large matrix faster (4096 x 24576, 8 rows: 14.8 us against 15.6 with two, 16 rows 17.2 / 19.2).
+    // A small one is faster with two, whose runs fill a deeper ring (2560 x 6144, 8 rows: 4.1 us against 4.8, 16 rows 5.7 / 6.2;
+    // 9728 x 2560 5.8 / 6.2, 7.9 / 8.4) - but up to eight rows three leave the next launch of a decode step more room (Qwen3-8B,
+    // five sequences: 50.2 ms for 24 steps against 53.1), so there only the ordered form does that.  32 rows need the registers
+    // of two.
+    r.occ = r.nt == 4 || (r.units * r.passes <= 800 && (ordered || r.nt == 2)) ? 2 : 3;
     const int slots = device_sm_count() * r.occ;
     r.run = int(((long long)r.units * r.passes + slots - 1) / slots);
     if (r.run < g_rows_min_run) r.run = g_rows_min_run;
@@ -361,9 +366,13 @@ int launch_rows(const RowsCall& call, const RowsPlan& plan, cudaStream_t stream)
 
 template <bool ORDERED>
 int launch_rows_nt(const RowsCall& call, const RowsPlan& plan, cudaStream_t stream) {
+    if constexpr (ORDERED) {
+        if (plan.nt == 1 && plan.occ == 2) return launch_rows<1, 5, 2, true>(call, plan, stream);
+    }
+    if (plan.nt == 2 && plan.occ == 2) return launch_rows<2, 4, 2, ORDERED>(call, plan, stream);
     if (plan.nt == 1) return launch_rows<1, 3, 3, ORDERED>(call, plan, stream);
     if (plan.nt == 2) return launch_rows<2, 3, 3, ORDERED>(call, plan, stream);
-    return launch_rows<4, 4, 2, ORDERED>(call, plan, stream);
+    return launch_rows<4, 3, 2, ORDERED>(call, plan, stream);
 }
 
 bool fill_rows(RowsCall& call, const RowsPlan& plan, const __half* x16, const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales,
@@ -396,7 +405,7 @@ int awq_rows_status() {
 // y += x16 . W (+ residual); y holds the addend.  Needs N % 32 == 0 and 16-byte aligned tensors.
 int awq_rows_launch(const __half* x16, const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales, float* y, const float* residual,
                     int M, int K, int N, cudaStream_t stream) {
-    const RowsPlan plan = plan_rows(M, K, N);
+    const RowsPlan plan = plan_rows(M, K, N, false);
     RowsCall call;
     if (!fill_rows(call, plan, x16, qweight, qzeros, scales, y, M, K, N)) {
         set_error("awq_gemm: tensor map encoding failed");
@@ -408,14 +417,14 @@ int awq_rows_launch(const __half* x16, const int32_t* qweight, const int32_t* qz
 
 // floats of the slots an ordered call writes
 size_t awq_rows_partial_floats(int M, int K, int N) {
-    const RowsPlan plan = plan_rows(M, K, N);
+    const RowsPlan plan = plan_rows(M, K, N, true);
     return size_t(plan.ctas + plan.tiles) * M * kTileCols;
 }
 
 // y = x16 . W (+ residual) with a fixed summation order; partial: awq_rows_partial_floats floats
 int awq_rows_ordered_launch(const __half* x16, const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales, float* y,
                             const float* residual, float* partial, int M, int K, int N, cudaStream_t stream) {
-    const RowsPlan plan = plan_rows(M, K, N);
+    const RowsPlan plan = plan_rows(M, K, N, true);
     RowsCall call;
     if (!fill_rows(call, plan, x16, qweight, qzeros, scales, y, M, K, N)) {
         set_error("awq_gemv: tensor map encoding failed");

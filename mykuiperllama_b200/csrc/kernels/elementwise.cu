@@ -315,7 +315,8 @@ int launch_rmsnorm(const float* x, const uint16_t* w, OUT* y, int M, int H, floa
 
 template <typename OUT>
 int launch_swiglu(float* gate_up, OUT* out, int M, int I, int clear_input, cudaStream_t stream, const char* what) {
-    if (I % 4 == 0 && ((reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0)
+    // a decode batch has too few elements for that: one per thread has the shorter chain
+    if (int64_t(M) * I >= int64_t(device_sm_count()) * 8192 && I % 4 == 0 && ((reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0)
         return pdl_status(launch_pdl(swiglu4_kernel<OUT>, dim3(grid_for(int64_t(M) * I / 4, 256)), dim3(256), 0, stream, gate_up, out, M, I / 4,
                                      clear_input), what);
     return pdl_status(launch_pdl(swiglu_kernel<OUT>, dim3(grid_for(int64_t(M) * I, 256)), dim3(256), 0, stream, gate_up, out, M, I, clear_input),
