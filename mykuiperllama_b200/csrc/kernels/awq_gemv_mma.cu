@@ -1220,6 +1220,14 @@ int awq_gemv_mma_launch(const float* x, const int32_t* qweight, const int32_t* q
     call.partial = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + head);
     const bool three = int_operand && rows == 1 && accumulate && g_int8_ctas == kCtasPerSmInt8 && call.U >= g_int8_ctas3_units;
     long long ctas = (long long)device_sm_count() * (three ? kCtasPerSmInt8 : kCtasPerSmMma);
+    // The last CTA of a column tile adds one slot per CTA that worked on it, eight in flight, so a small matrix cut into single
+    // units waits for its slots: runs of a whole quantisation group where there are enough of them, of two units below that
+    // (2048 x 2048, 128 units: 7.8 us with runs of one, 6.4 two, 7.0 four; 2560 x 2560, 240 units: 8.9 / 7.7 / 7.2; 4096 x
+    // 4096 10.2 / 9.3 / 8.8; 12288 x 1024 19.7 / 14.3 / 11.5; from 1536 units on the runs are longer anyway).
+    if (!accumulate) {
+        const long long run = call.U < 240 ? 2 : 4;
+        if (ctas * run > call.U) ctas = (call.U + run - 1) / run;
+    }
     if (ctas > call.U) ctas = call.U;
     if ((norm_w || swiglu) && !accumulate) {
         set_error("awq_gemv_mma: the fused input norm / SwiGLU exist in accumulate mode only");
