@@ -22,7 +22,8 @@ def _ptr(t):
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    # the raw handle of torch.cuda.current_stream(), without building a Stream object for every call (3.2 us of a 10 us call)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _dev(*ts):
