@@ -128,6 +128,11 @@ __device__ __forceinline__ uint32_t bf16_round_bits(float v) {  // round to near
 __global__ void __launch_bounds__(kMmaThreads, 1)
 bf16_rows_mma_kernel(const float* x, const uint16_t* __restrict__ W, float* y, int M, int K, int N) {
     extern __shared__ __align__(16) unsigned char planes[];  // [3 planes][8 rows][2 K + 64 bytes]
+    // eight token rows per blockIdx.y
+    const int m_first = int(blockIdx.y) * kMmaRows;
+    x += size_t(m_first) * K;
+    y += size_t(m_first) * N;
+    M = min(M - m_first, kMmaRows);
     const int row_bytes = 2 * K + 64;  // the 64 bytes stagger the rows over the banks (16-byte reads of a quarter warp)
     const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
     const int warp_global = blockIdx.x * (kMmaThreads / 32) + (threadIdx.x >> 5);
@@ -203,18 +208,23 @@ int g_bf16_mma = 1;  // tuning key "bf16_mma": 0 keeps every call on the SIMT ke
 
 size_t mma_smem_bytes(int K) { return size_t(3 * kMmaRows) * size_t(2 * K + 64); }
 
+// Up to four blocks of eight rows run side by side, each on its share of the SMs: they walk the weight rows at the same
+// pace, so that one reads them from memory and the others from the L2.
+constexpr int kMmaBlocks = 4;
+
 int launch_mma_rows(const float* x, const uint16_t* W, float* y, int M, int K, int N, cudaStream_t stream) {
+    const int blocks = (M + kMmaRows - 1) / kMmaRows;
     const size_t smem = mma_smem_bytes(K);
     static size_t configured[kMaxDevices] = {};
     if (!ensure_dynamic_smem(bf16_rows_mma_kernel, smem, configured)) {
         set_error("bf16_gemv: cannot reserve %zu bytes of shared memory", smem);
         return KUIPER_INTERNAL_ERROR;
     }
-    int grid = device_sm_count();
+    int grid = device_sm_count() / blocks;
     const int groups = (N + 15) / 16, per_cta = kMmaThreads / 32;
     if (grid > (groups + per_cta - 1) / per_cta) grid = (groups + per_cta - 1) / per_cta;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.gridDim = dim3(grid, blocks, 1);
     cfg.blockDim = dim3(kMmaThreads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -252,8 +262,8 @@ extern "C" int kuiper_bf16_gemv_f32(const float* x, const uint16_t* W, float* y,
     cudaStream_t st = as_stream(stream);
     // three rows or more: passes of up to eight rows on the tensor cores (K in whole 32-column steps, planes in shared memory)
     if (g_bf16_mma && M >= 3 && K % 32 == 0 && mma_smem_bytes(K) <= 220 * 1024) {
-        for (int m0 = 0; m0 < M; m0 += kMmaRows) {
-            const int rows = M - m0 < kMmaRows ? M - m0 : kMmaRows;
+        for (int m0 = 0; m0 < M; m0 += kMmaBlocks * kMmaRows) {
+            const int rows = M - m0 < kMmaBlocks * kMmaRows ? M - m0 : kMmaBlocks * kMmaRows;
             const int rc = launch_mma_rows(x + size_t(m0) * K, W, y + size_t(m0) * N, rows, K, N, st);
             if (rc != KUIPER_OK) return rc;
         }
