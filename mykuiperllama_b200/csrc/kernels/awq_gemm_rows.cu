@@ -15,7 +15,9 @@
 // Work: units of 128 weight rows x 256 columns (16 KB, one quantisation group), numbered column tile major, dealt in
 // equal contiguous runs.  A CTA is four consumer warps of 64 columns each and a producer warp that keeps a ring of
 // stages full (four TMA boxes of 32 rows, the group's zero words and scales, the token rows' 128 fp16 activations,
-// rows 272 bytes apart so that ldmatrix is conflict-free).  A run that leaves a column tile adds its sums to y with
+// rows 272 bytes apart so that ldmatrix is conflict-free).  Up to eight rows may come as fp32, or as gate|up rows whose
+// SwiGLU is the operand: two more warps then read them and write the fp16 stage, in turns, which saves a launch of 2 to 3 us
+// before a projection of 4 to 10 us.  A run that leaves a column tile adds its sums to y with
 // reductions, or, where the caller needs a fixed order, writes them to a workspace slot that a second kernel adds up
 // in run order.  More than 32 rows run as passes over the same weights (grid.y), which the L2 serves.
 #include <cuda.h>
@@ -39,6 +41,8 @@ constexpr int kScaleBytesR = kTileCols * 2;
 constexpr int kXPitch = kGroupRows * 2 + 16;
 constexpr int kConsumerWarps = 4;
 constexpr int kThreadsRows = (kConsumerWarps + 1) * 32;
+enum RowsOperand { kRowsF16, kRowsF32, kRowsSwiglu };
+constexpr int rows_threads(int operand) { return kThreadsRows + (operand == kRowsF16 ? 0 : 64); }
 constexpr uint32_t kSpinLimitRows = 1u << 22;
 
 __device__ int g_rows_wait_error = 0;
@@ -46,6 +50,7 @@ __device__ int g_rows_wait_error = 0;
 struct RowsCall {
     CUtensorMap tmap;
     const __half* x;        // [M, K]
+    const float* x32;       // the other operands: [M, K], or [M, 2 K] gate|up rows
     const uint32_t* qz;     // [K/128, N/8]
     const __half* scales;   // [K/128, N]
     float* y;               // [M, N]
@@ -93,8 +98,8 @@ __device__ __forceinline__ void rows_mma(float (&d)[4], uint32_t a0, uint32_t a1
 template <int NT>
 constexpr int rows_aux_bytes() { return kZeroBytesR + kScaleBytesR + 8 * NT * kXPitch; }
 
-template <int NT, int STAGES, int OCC, bool ORDERED>
-__global__ void __launch_bounds__(kThreadsRows, OCC) awq_rows_kernel(const __grid_constant__ RowsCall p) {
+template <int NT, int STAGES, int OCC, bool ORDERED, int OPERAND>
+__global__ void __launch_bounds__(rows_threads(OPERAND), OCC) awq_rows_kernel(const __grid_constant__ RowsCall p) {
     extern __shared__ unsigned char smem_raw[];
     const uint32_t smem = (rsm(smem_raw) + 1023u) & ~1023u;
     __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES];
@@ -110,7 +115,7 @@ __global__ void __launch_bounds__(kThreadsRows, OCC) awq_rows_kernel(const __gri
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int i = 0; i < STAGES; i++) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(rsm(&full_bar[i])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(rsm(&full_bar[i])), "n"(OPERAND == kRowsF16 ? 1 : 2));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(rsm(&empty_bar[i])), "n"(kConsumerWarps));
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -128,7 +133,7 @@ __global__ void __launch_bounds__(kThreadsRows, OCC) awq_rows_kernel(const __gri
                 const uint32_t zbytes = uint32_t(cols) >> 1, sbytes = uint32_t(cols) * 2;
                 const uint32_t bar = rsm(&full_bar[s]), w = smem + s * kWeightBytes, aux = aux0 + s * kAux;
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                             "r"(uint32_t(kWeightBytes) + zbytes + sbytes + uint32_t(rows) * kGroupRows * 2)
+                             "r"(uint32_t(kWeightBytes) + zbytes + sbytes + (OPERAND == kRowsF16 ? uint32_t(rows) * kGroupRows * 2 : 0u))
                              : "memory");
 #pragma unroll
                 for (int b = 0; b < kGroupRows / kBoxRows; b++)
@@ -143,6 +148,7 @@ __global__ void __launch_bounds__(kThreadsRows, OCC) awq_rows_kernel(const __gri
             __syncwarp();
         };
         auto issue_x = [&](int i, int s) {
+            if constexpr (OPERAND != kRowsF16) return;
             const int u = u0 + i, group = u % p.groups;
             if (lane < rows)
                 rows_bulk(aux0 + s * kAux + kZeroBytesR + kScaleBytesR + lane * kXPitch,
@@ -152,7 +158,7 @@ __global__ void __launch_bounds__(kThreadsRows, OCC) awq_rows_kernel(const __gri
         // the weights do not depend on the preceding kernel, the activations do
         const int ahead = min(STAGES, n_units);
         for (int i = 0; i < ahead; i++) issue_weights(i, i);
-        pdl_wait();
+        if constexpr (OPERAND == kRowsF16) pdl_wait();
         for (int i = 0; i < ahead; i++) issue_x(i, i);
         for (int i = ahead; i < n_units; i++) {
             const int s = i % STAGES;
@@ -166,6 +172,46 @@ __global__ void __launch_bounds__(kThreadsRows, OCC) awq_rows_kernel(const __gri
             issue_x(i, s);
         }
         return;
+    }
+
+    if constexpr (OPERAND != kRowsF16) {
+        if (warp > kConsumerWarps) {
+            // -------------------------------------------------------- fp32 rows: the two warps take alternate stages
+            pdl_wait();
+            for (int i = warp - kConsumerWarps - 1; i < n_units; i += 2) {
+                const int s = i % STAGES, group = (u0 + i) % p.groups;
+                float4 v[8 * NT];
+#pragma unroll
+                for (int r = 0; r < 8 * NT; r++) {
+                    const int m = m0 + min(r, rows - 1);
+                    if constexpr (OPERAND == kRowsSwiglu) {
+                        const float* src = p.x32 + size_t(m) * 2 * p.K + group * kGroupRows + lane * 4;
+                        const float4 g = __ldcg(reinterpret_cast<const float4*>(src)), u = __ldcg(reinterpret_cast<const float4*>(src + p.K));
+                        v[r] = make_float4((g.x / (1.0f + expf(-g.x))) * u.x, (g.y / (1.0f + expf(-g.y))) * u.y,
+                                           (g.z / (1.0f + expf(-g.z))) * u.z, (g.w / (1.0f + expf(-g.w))) * u.w);
+                    } else {
+                        v[r] = __ldcg(reinterpret_cast<const float4*>(p.x32 + size_t(m) * p.K + group * kGroupRows + lane * 4));
+                    }
+                }
+                // a warp sees every other stage of the ring; the wait on the parity is safe because the consumers free the stages
+                // in order and this warp has seen the stage before last filled
+                if (i >= STAGES && !rows_wait(rsm(&empty_bar[s]), uint32_t(i / STAGES - 1) & 1u, true)) {
+                    if (lane == 0) atomicExch(&g_rows_wait_error, 13);
+                    return;
+                }
+                const uint32_t dst = aux0 + s * kAux + kZeroBytesR + kScaleBytesR + lane * 8;
+#pragma unroll
+                for (int r = 0; r < 8 * NT; r++) {
+                    const __half2 a = __floats2half2_rn(v[r].x, v[r].y), b = __floats2half2_rn(v[r].z, v[r].w);
+                    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst + r * kXPitch), "r"(*reinterpret_cast<const uint32_t*>(&a)),
+                                 "r"(*reinterpret_cast<const uint32_t*>(&b))
+                                 : "memory");
+                }
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(rsm(&full_bar[s])) : "memory");
+            }
+            return;
+        }
     }
 
     // ---------------------------------------------------------------- consumers: 64 columns each
@@ -352,27 +398,32 @@ RowsPlan plan_rows(int M, int K, int N, bool ordered) {
     return r;
 }
 
-template <int NT, int STAGES, int OCC, bool ORDERED>
+template <int NT, int STAGES, int OCC, bool ORDERED, int OPERAND>
 int launch_rows(const RowsCall& call, const RowsPlan& plan, cudaStream_t stream) {
-    auto kern = awq_rows_kernel<NT, STAGES, OCC, ORDERED>;
+    auto kern = awq_rows_kernel<NT, STAGES, OCC, ORDERED, OPERAND>;
     const size_t smem = 1024 + size_t(STAGES) * (kWeightBytes + rows_aux_bytes<NT>());
     static size_t configured[kMaxDevices] = {};
     if (!ensure_dynamic_smem(kern, smem, configured)) {
         set_error("awq_gemm: cannot reserve %zu bytes of shared memory", smem);
         return KUIPER_INTERNAL_ERROR;
     }
-    return pdl_status(launch_pdl(kern, dim3(plan.ctas, plan.passes), dim3(kThreadsRows), smem, stream, call), "awq_gemm rows");
+    return pdl_status(launch_pdl(kern, dim3(plan.ctas, plan.passes), dim3(rows_threads(OPERAND)), smem, stream, call), "awq_gemm rows");
 }
 
 template <bool ORDERED>
-int launch_rows_nt(const RowsCall& call, const RowsPlan& plan, cudaStream_t stream) {
+int launch_rows_nt(const RowsCall& call, const RowsPlan& plan, int operand, cudaStream_t stream) {
+    if (operand == kRowsSwiglu) return launch_rows<1, 3, 3, false, kRowsSwiglu>(call, plan, stream);
     if constexpr (ORDERED) {
-        if (plan.nt == 1 && plan.occ == 2) return launch_rows<1, 5, 2, true>(call, plan, stream);
+        if (operand == kRowsF32 && plan.occ == 2) return launch_rows<1, 5, 2, true, kRowsF32>(call, plan, stream);
     }
-    if (plan.nt == 2 && plan.occ == 2) return launch_rows<2, 4, 2, ORDERED>(call, plan, stream);
-    if (plan.nt == 1) return launch_rows<1, 3, 3, ORDERED>(call, plan, stream);
-    if (plan.nt == 2) return launch_rows<2, 3, 3, ORDERED>(call, plan, stream);
-    return launch_rows<4, 3, 2, ORDERED>(call, plan, stream);
+    if (operand == kRowsF32) return launch_rows<1, 3, 3, ORDERED, kRowsF32>(call, plan, stream);
+    if constexpr (ORDERED) {
+        if (plan.nt == 1 && plan.occ == 2) return launch_rows<1, 5, 2, true, kRowsF16>(call, plan, stream);
+    }
+    if (plan.nt == 2 && plan.occ == 2) return launch_rows<2, 4, 2, ORDERED, kRowsF16>(call, plan, stream);
+    if (plan.nt == 1) return launch_rows<1, 3, 3, ORDERED, kRowsF16>(call, plan, stream);
+    if (plan.nt == 2) return launch_rows<2, 3, 3, ORDERED, kRowsF16>(call, plan, stream);
+    return launch_rows<4, 3, 2, ORDERED, kRowsF16>(call, plan, stream);
 }
 
 bool fill_rows(RowsCall& call, const RowsPlan& plan, const __half* x16, const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales,
@@ -412,7 +463,23 @@ int awq_rows_launch(const __half* x16, const int32_t* qweight, const int32_t* qz
         return KUIPER_INTERNAL_ERROR;
     }
     call.residual = residual;
-    return launch_rows_nt<false>(call, plan, stream);
+    return launch_rows_nt<false>(call, plan, kRowsF16, stream);
+}
+
+// most rows of awq_rows_f32_launch
+int awq_rows_f32_max() { return 8; }
+
+// y += op(x) . W for fp32 rows; op: fp16 rounding, or (swiglu) silu(gate) * up of [M, 2 K] rows rounded to fp16
+int awq_rows_f32_launch(const float* x, bool swiglu, const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales, float* y, int M, int K,
+                        int N, cudaStream_t stream) {
+    const RowsPlan plan = plan_rows(M, K, N, false);
+    RowsCall call;
+    if (!fill_rows(call, plan, nullptr, qweight, qzeros, scales, y, M, K, N)) {
+        set_error("awq_gemv: tensor map encoding failed");
+        return KUIPER_INTERNAL_ERROR;
+    }
+    call.x32 = x;
+    return launch_rows_nt<false>(call, plan, swiglu ? kRowsSwiglu : kRowsF32, stream);
 }
 
 // floats of the slots an ordered call writes
@@ -421,8 +488,9 @@ size_t awq_rows_partial_floats(int M, int K, int N) {
     return size_t(plan.ctas + plan.tiles) * M * kTileCols;
 }
 
-// y = x16 . W (+ residual) with a fixed summation order; partial: awq_rows_partial_floats floats
-int awq_rows_ordered_launch(const __half* x16, const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales, float* y,
+// y = x . W (+ residual) with a fixed summation order, x as fp16 (x16) or, up to awq_rows_f32_max rows, fp32; partial:
+// awq_rows_partial_floats floats
+int awq_rows_ordered_launch(const __half* x16, const float* x32, const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales, float* y,
                             const float* residual, float* partial, int M, int K, int N, cudaStream_t stream) {
     const RowsPlan plan = plan_rows(M, K, N, true);
     RowsCall call;
@@ -431,7 +499,8 @@ int awq_rows_ordered_launch(const __half* x16, const int32_t* qweight, const int
         return KUIPER_INTERNAL_ERROR;
     }
     call.partial = partial;
-    const int rc = launch_rows_nt<true>(call, plan, stream);
+    call.x32 = x32;
+    const int rc = launch_rows_nt<true>(call, plan, x32 ? kRowsF32 : kRowsF16, stream);
     if (rc != KUIPER_OK) return rc;
     return pdl_status(launch_pdl(awq_rows_combine_kernel, dim3((N / 4 + 63) / 64, M), dim3(64), 0, stream, static_cast<const float*>(partial), residual, y,
                                  M, N, plan.groups, plan.run),

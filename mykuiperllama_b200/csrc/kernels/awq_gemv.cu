@@ -428,7 +428,10 @@ bool awq_gemv_mma_supported(int K, int N);
 int awq_gemv_mma_status();
 int awq_gemv_mma_max_rows(bool accumulate);
 size_t awq_rows_partial_floats(int M, int K, int N);
-int awq_rows_ordered_launch(const __half* x16, const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales, float* y,
+int awq_rows_f32_max();
+int awq_rows_f32_launch(const float* x, bool swiglu, const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales, float* y, int M, int K,
+                        int N, cudaStream_t stream);
+int awq_rows_ordered_launch(const __half* x16, const float* x32, const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales, float* y,
                             const float* residual, float* partial, int M, int K, int N, cudaStream_t stream);
 int awq_rows_status();
 int convert_f16_launch(const float* x, __half* out, int64_t n4, float* zero, int64_t zero4, cudaStream_t stream);
@@ -503,9 +506,12 @@ extern "C" int kuiper_awq_gemv_f32(const float* x, const int32_t* qweight, const
         if (mma && M >= g_rows_min && workspace != nullptr && workspace_bytes >= gemv_rows_workspace_bytes(M, K, N) &&
             ((reinterpret_cast<uintptr_t>(workspace) | reinterpret_cast<uintptr_t>(x)) & 15) == 0) {
             __half* x16 = reinterpret_cast<__half*>(static_cast<char*>(workspace) + gemv_rows_x16(M, K, N));
-            const int rc = convert_f16_launch(x, x16, int64_t(M) * K / 4, nullptr, 0, st);
-            if (rc != KUIPER_OK) return rc;
-            return awq_rows_ordered_launch(x16, qweight, qzeros, scales, y, residual,
+            const bool direct = M <= awq_rows_f32_max();  // the kernel rounds the rows itself
+            if (!direct) {
+                const int rc = convert_f16_launch(x, x16, int64_t(M) * K / 4, nullptr, 0, st);
+                if (rc != KUIPER_OK) return rc;
+            }
+            return awq_rows_ordered_launch(direct ? nullptr : x16, direct ? x : nullptr, qweight, qzeros, scales, y, residual,
                                            reinterpret_cast<float*>(static_cast<char*>(workspace) + gemv_rows_head(N)), M, K, N, st);
         }
         KUIPER_REQUIRE(workspace != nullptr && workspace_bytes >= awq_gemv_tma_workspace_bytes(K, N),
@@ -584,6 +590,12 @@ static int awq_gemv_accum_common(const float* x, const uint16_t* norm_w, float e
     // share the counters and are dealt out statically)
     // the integer operand is a one-row kernel: it serves single-row calls, everything else rounds to fp16
     const bool int_operand = act_mode == KUIPER_ACT_INT16_BLOCK && M == 1 && mma;
+    // three rows and more without a norm: one pass over the weights (eight rows of 4096 x 24576 14.8 us against two passes of
+    // four 28.2, five rows of 9728 x 2560 5.5 / 13.8).  The engine's decode steps take fp16 rows from a separate launch from
+    // three rows on: the wider CTAs of this form leave the next launch less room (Qwen3-8B, five sequences: 51.8 to 53.1 ms
+    // against 50.5).
+    if (mma && norm_w == nullptr && M >= 3 && M <= awq_rows_f32_max())
+        return awq_rows_f32_launch(x, swiglu, qweight, qzeros, scales, y, M, K, N, st);
     const int max_rows = mma ? awq_gemv_mma_max_rows(true) : 2;
     for (int m0 = 0; m0 < M;) {
         const int mt = (M - m0 >= max_rows) ? max_rows : (M - m0);

@@ -57,6 +57,21 @@ def test_few_rows(cuda, M, K, N):
         assert _err(y, r) <= TOL, (i, _err(y, r))
 
 
+@pytest.mark.parametrize("M,K,N", [(2, 128, 32), (3, 2560, 6144), (5, 12288, 4096), (8, 640, 288)])
+def test_fp32_and_gate_up_operands(cuda, M, K, N):
+    x, w, ref = _case(M, K, N, M + K + N)
+    res = torch.randn((M, N), device="cuda")
+    assert _err(cuda.awq_gemv_accum(x, *w, res.clone()), ref + res.double()) <= TOL
+    # SwiGLU of gate|up rows, rounded to fp16, is the operand: the same as the separate kernel followed by the product
+    gate_up = torch.randn((M, 2 * K), device="cuda")
+    operand = cuda.swiglu_f16(gate_up)
+    got = cuda.swiglu_awq_gemv_accum(gate_up, *w, res.clone())
+    want = cuda.awq_gemm_f16in(operand, *w, y=res.clone(), accumulate=True)
+    torch.cuda.synchronize()
+    cuda.awq_gemv_status()
+    assert _err(got, want.double()) <= TOL
+
+
 def test_rows_beyond_the_matrix_stay_untouched(cuda):
     x, w, ref = _case(5, 256, 96, 3)
     y = torch.full((9, 96), 7.0, device="cuda")
