@@ -68,7 +68,7 @@ KUIPER_API int kuiper_awq_unpack_u8(const int32_t* qweight, uint8_t* out, int K,
 /* fp32 dequantisation W[K,N] = (q - z) * s, exact */
 KUIPER_API int kuiper_awq_dequant_f32(const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales,
                            float* W, int K, int N, int group, kuiper_stream_t stream);
-/* bf16 dequantisation (round to nearest even) used by the M>=16 tensor-core path */
+/* bf16 dequantisation (round to nearest even) */
 KUIPER_API int kuiper_awq_dequant_bf16(const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales,
                             uint16_t* W, int K, int N, int group, kuiper_stream_t stream);
 
@@ -176,18 +176,21 @@ KUIPER_API int kuiper_awq_gemv_f32_noalloc(const float* x, const int32_t* qweigh
                                            const uint16_t* scales, float* y, const float* residual,
                                            int M, int K, int N, int group, kuiper_stream_t stream);
 
-/* ---- INT4-AWQ GEMM on the tcgen05 tensor cores, for M >= 16 token rows (prefill, batched decode).
- * Same placeholder as the GEMV (kuiper/include/op/matmul.h:1-11).  x is rounded to fp16, the weight
- * (q - z) * s is rounded to fp16, accumulation is fp32 in tensor memory.
+/* ---- INT4-AWQ GEMM for several token rows (prefill, batched decode).
+ * Same placeholder as the GEMV (kuiper/include/op/matmul.h:1-11).  x is rounded to fp16.  Up to 32 rows (N % 32 == 0) the
+ * products are exact (packed-word kernel on mma.sync); beyond that the weight (q - z) * s is rounded to fp16 and the product
+ * runs on the tcgen05 tensor cores, accumulation in fp32.
  *   accumulate == 0, residual == NULL : y  = x . W
  *   accumulate == 0, residual != NULL : y  = x . W + residual   (residual may alias y)
- *   accumulate != 0                   : y += x . W
- * A launch with few output tiles (M <= 128 or so) splits K over several CTAs per tile, which add their sums with
- * reductions: the summation order is then not fixed (differences ~1e-6); larger launches are deterministic.
- * Any M > 0 is accepted (rows are padded to 128 inside the kernel); K % 128 == 0, N % 8 == 0.
- * workspace: kuiper_awq_gemm_workspace_bytes(M, K) bytes (16-byte aligned) for the fp16 copy of x that the
- * pipelined kernel reads (128 x 256 tiles); required.
- * kuiper_awq_gemm_status() synchronously reads the kernel's bounded-wait error word. ---- */
+ *   accumulate == 1                   : y += x . W
+ * A launch with few output tiles (up to 32 rows, or ceil(M / 128) * ceil(N / 256) below 4/3 of two CTAs per SM) splits K over
+ * several CTAs, which add their sums with reductions: the summation order is then not fixed (differences ~1e-6); larger
+ * launches are deterministic, unless accumulate has KUIPER_GEMM_ANY_ORDER set, which lets them share tiles as well.
+ * Any M > 0 is accepted; K % 128 == 0, N % 8 == 0.
+ * workspace: kuiper_awq_gemm_workspace_bytes(M, K) bytes (16-byte aligned) for the fp16 copy of x that the kernels read;
+ * required.
+ * kuiper_awq_gemm_status() synchronously reads the kernels' bounded-wait error words. ---- */
+#define KUIPER_GEMM_ANY_ORDER 2
 KUIPER_API size_t kuiper_awq_gemm_workspace_bytes(int M, int K);
 KUIPER_API int kuiper_awq_gemm_f32(const float* x, const int32_t* qweight, const int32_t* qzeros,
                                    const uint16_t* scales, float* y, const float* residual, int accumulate,

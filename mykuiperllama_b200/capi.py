@@ -161,7 +161,7 @@ def awq_gemm_workspace(M, K, device="cuda"):
 
 
 def awq_gemm(x, qweight, qzeros, scales, y=None, residual=None, accumulate=False, group=128, workspace="auto"):
-    """Tensor-core INT4 GEMM for M >= 16 rows: y = x . W (+ residual), or y += x . W.
+    """INT4 GEMM for several rows: y = x . W (+ residual), or y += x . W.
     workspace: "auto" allocates the fp16 activation copy the kernel reads; a tensor is used as it is."""
     _dev(x, qweight, qzeros, scales)
     M, K = x.shape

@@ -1,8 +1,11 @@
-// INT4-AWQ GEMM on the 5th-generation tensor cores (tcgen05 + TMEM) for M >= 16 token rows:
+// INT4-AWQ GEMM on the 5th-generation tensor cores (tcgen05 + TMEM) for calls of many token rows:
 // prefill chunks and batched decode, where the operation is a dense contraction.
 // Same placeholder as the GEMV: kuiper/include/op/matmul.h:1-11 of the reference.
 //
 // y[M,N] (+)= x[M,K] . dequant(qweight)[K,N]
+//
+// Calls of up to 32 rows go to awq_gemm_rows.cu, others to the 256 x 256 tiles of awq_gemm_tc4_kernel further down; the two
+// kernels described first remain for what those do not take (N % 32 != 0, no K split wanted, see tiles_pay).
 //
 // One CTA owns a 128 x 256 output tile; its fp32 accumulator lives in tensor memory (128 lanes x 256
 // columns), two CTAs share an SM.  The activations are converted to fp16 once per call (the same operand
@@ -13,8 +16,8 @@
 // store.  Both operands are stored K-major with the 128-byte swizzle: a tile row is the 64 K values (128
 // bytes) of one token row / weight column, eight rows form a 1024-byte atom, and the 16-byte chunk c of row
 // r sits at chunk position c ^ (r % 8).  One thread issues four tcgen05.mma (K = 16 each) per stage and a
-// tcgen05.commit onto the stage's mbarrier; a stage is refilled only after that commit.  In the default kernel
-// (awq_gemm_tc3_kernel) that thread belongs to a warp of its own and learns through a second mbarrier that the
+// tcgen05.commit onto the stage's mbarrier; a stage is refilled only after that commit.  In
+// awq_gemm_tc3_kernel that thread belongs to a warp of its own and learns through a second mbarrier that the
 // producer warps have filled the stage; awq_gemm_tc2_kernel hands the stage over at a block-wide barrier.  The
 // epilogue reads the accumulator with tcgen05.ld (one TMEM lane = one output row per thread).
 //
@@ -970,8 +973,9 @@ __global__ void __launch_bounds__(256) zero_split_kernel(float4* y, int M, int N
     for (int i = (m >= row0 ? 0 : col4) + threadIdx.x; i < N4; i += 256) y[size_t(m) * N4 + i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// y[add ? += : =] x16 . W (+ residual)
-int launch_tiles4(const GemmParams& g, const __half* x16, cudaStream_t stream) {
+// y[add ? += : =] x16 . W (+ residual); share: tiles may be added up from several CTAs, otherwise every tile is one CTA's (a fixed
+// order of the sums, at the price of a partial last wave)
+int launch_tiles4(const GemmParams& g, const __half* x16, bool share, bool zeroed, cudaStream_t stream) {
     GemmCall4 c;
     memset(&c, 0, sizeof(c));
     if (!encode_rows_map(&c.x_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x16, g.M, g.K, kBK, kBM, CU_TENSOR_MAP_SWIZZLE_128B) ||
@@ -993,12 +997,16 @@ int launch_tiles4(const GemmParams& g, const __half* x16, cudaStream_t stream) {
     const int split_units = c.full_units - c.whole_tiles * ctas * c.groups;
     c.full_run = (split_units + ctas - 1) / ctas;
     c.tail_run = (c.tail_units + ctas - 1) / ctas;
+    if (!share) {  // runs of whole tiles
+        c.full_run = (c.full_run + c.groups - 1) / c.groups * c.groups;
+        c.tail_run = (c.tail_run + c.groups - 1) / c.groups * c.groups;
+    }
     static size_t configured[kMaxDevices] = {};
     if (!ensure_dynamic_smem(awq_gemm_tc4_kernel, kSmem4, configured)) {
         set_error("awq_gemm: cannot reserve %zu bytes of shared memory", kSmem4);
         return KUIPER_INTERNAL_ERROR;
     }
-    if (!c.add && (split_units > 0 || tail)) {
+    if (!c.add && share && !zeroed && (split_units > 0 || tail)) {
         const int full_rows = c.m_tiles - tail;
         const int first_col = split_units > 0 ? c.whole_tiles * ctas / full_rows * kTileN4 : g.N;  // the first column tile that is not whole
         const int rc = pdl_status(launch_pdl(zero_split_kernel, dim3(g.M), dim3(256), 0, stream, reinterpret_cast<float4*>(g.y), g.M, g.N / 4,
@@ -1064,6 +1072,8 @@ extern "C" size_t kuiper_awq_gemm_workspace_bytes(int M, int K) {
 static int gemm_common(const float* x, const __half* x16_in, const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales,
                        float* y, const float* residual, int accumulate, int M, int K, int N, int group, void* workspace,
                        size_t workspace_bytes, kuiper_stream_t stream) {
+    const bool any_order = (accumulate & KUIPER_GEMM_ANY_ORDER) != 0;
+    accumulate &= ~KUIPER_GEMM_ANY_ORDER;
     KUIPER_REQUIRE((x || x16_in) && qweight && qzeros && scales && y, "awq_gemm: null tensor pointer");
     KUIPER_REQUIRE(M > 0 && K > 0 && N > 0, "awq_gemm: empty shape M=%d K=%d N=%d", M, K, N);
     KUIPER_REQUIRE(group == 128, "awq_gemm: group size %d is not supported (128 only)", group);
@@ -1112,11 +1122,14 @@ static int gemm_common(const float* x, const __half* x16_in, const int32_t* qwei
     }
     if (g_gemm_impl == 3 && g_gemm_split_k == 1 && g_gemm_tile_rows > 0 && M >= g_gemm_tile_rows && encode_fn_tc() != nullptr &&
         tiles_pay(M, int(grid2.x * grid2.y), splits)) {
+        const bool share = any_order || splits > 1;
+        // where no tile is whole, the launch that converts the activations zeroes y as well
+        const bool zero_all = share && n4 > 0 && p.mode != 2 && (M / kTileM4) * ((N + kTileN4 - 1) / kTileN4) < device_sm_count();
         if (n4 > 0) {
-            const int rc = convert_f16_launch(x, x16_ws, n4, nullptr, 0, as_stream(stream));
+            const int rc = convert_f16_launch(x, x16_ws, n4, y, zero_all ? int64_t(M) * N / 4 : 0, as_stream(stream));
             if (rc != KUIPER_OK) return rc;
         }
-        return launch_tiles4(p, x16_in ? x16_in : x16_ws, as_stream(stream));
+        return launch_tiles4(p, x16_in ? x16_in : x16_ws, share, zero_all, as_stream(stream));
     }
     const bool zero_y = splits > 1 && p.mode != 2;
     // activations converted to fp16 once (the same launch zeroes y for a split call), then 128 x 256 output tiles

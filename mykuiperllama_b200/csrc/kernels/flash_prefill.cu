@@ -1,6 +1,6 @@
 // Causal attention for a prompt chunk: M consecutive token rows of ONE sequence against the bf16 KV cache (which already
 // holds the chunk's own rows), tiled so that every K / V tile is loaded once per block of query rows instead of once
-// per row.  Fills the same placeholder as the decode kernel (kuiper/include/op/mha.h:1-11 of the reference).
+// per row.  Larger chunks take the kernel of flash_prefill_tc.cu.  Fills the same placeholder as the decode kernel (kuiper/include/op/mha.h:1-11 of the reference).
 //
 // Grid (ceil(M / BR), Nkv): a CTA owns BR = 64 / R consecutive query rows of one kv head, i.e. 64 query vectors
 // (row, head) with R = Nq / Nkv heads per kv head; warp w owns vectors 16w .. 16w+15 (vector v = row * R + head).

@@ -41,7 +41,7 @@ public:
     // no fused prologue ([max rows, dim1] fp32)
     void set_norm_scratch(const tensor::Tensor& scratch) { norm_scratch_ = scratch; }
     // quantised layers, fp16-operand mode: inputs of at least this many rows go to the GEMM entry (packed-word kernel up to
-    // about a hundred rows, tcgen05 tiles beyond) instead of the GEMV in passes of four rows (0 = never).  One pass of the
+    // 32 rows, tcgen05 tiles beyond) instead of the GEMV in passes of four rows (0 = never).  One pass of the
     // GEMV also runs the input norm / SwiGLU itself, which saves four launches a layer: Qwen3-8B decode of two sequences
     // takes the same time either way (1.82 ms a step, 0.6B 0.71 against 0.82), of three 1.97 against 2.13, of five
     // 2.00 against 3.35.

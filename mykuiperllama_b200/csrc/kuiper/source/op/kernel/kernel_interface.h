@@ -41,7 +41,7 @@ using MatmulKernelQuantAccum = void (*)(const tensor::Tensor& input, const tenso
                                         const tensor::Tensor* input_norm_weight, float eps, bool input_swiglu,
                                         int32_t act_mode, const tensor::Tensor* tickets, void* stream);
 
-// Tensor-core path for M >= 16 rows: output = input . dequant(...) (+ residual), or output += ... when accumulate.
+// Path for several rows: output = input . dequant(...) (+ residual), or output += ... when accumulate.
 using MatmulKernelQuantGemm = void (*)(const tensor::Tensor& input, const tensor::Tensor& qweight,
                                        const tensor::Tensor& qzeros, const tensor::Tensor& scales,
                                        const tensor::Tensor& output, const tensor::Tensor* residual, bool accumulate,

@@ -13,7 +13,7 @@ TOL = 1e-3
 
 
 @pytest.mark.parametrize("M,K,N", [(129, 128, 8), (200, 256, 264), (256, 2560, 2560), (257, 1152, 1000), (333, 4096, 1536), (384, 128, 520),
-                                   (512, 640, 6144), (700, 384, 256), (1025, 1024, 2080)])
+                                   (512, 640, 6144), (700, 384, 256), (1025, 1024, 2080), (1153, 256, 12320)])
 def test_many_rows(cuda, M, K, N):  # noqa: F811
     x, w, ref = _case(M, K, N, M + K + N)
     res = torch.randn((M, N), device="cuda")
@@ -31,4 +31,6 @@ def test_many_rows(cuda, M, K, N):  # noqa: F811
     assert bool((guard[M:] == 7.0).all())
     for i, (y, r) in enumerate(outs):
         assert _err(y, r) <= TOL, (i, _err(y, r))
+    if -(-M // 128) * -(-N // 256) >= 400:  # the fixed order of a launch with many tiles
+        assert torch.equal(outs[0][0], cuda.awq_gemm(x, *w)) and torch.equal(outs[2][0], outs[3][0])
     assert _err(outs[0][0], other.double()) <= 1e-5  # fp32 sums of up to 4096 products in two orders
