@@ -182,15 +182,14 @@ KUIPER_API int kuiper_awq_gemv_f32_noalloc(const float* x, const int32_t* qweigh
  * runs on the tcgen05 tensor cores, accumulation in fp32.
  *   accumulate == 0, residual == NULL : y  = x . W
  *   accumulate == 0, residual != NULL : y  = x . W + residual   (residual may alias y)
- *   accumulate == 1                   : y += x . W
+ *   accumulate != 0                   : y += x . W
  * A launch with few output tiles (up to 32 rows, or ceil(M / 128) * ceil(N / 256) below 4/3 of two CTAs per SM) splits K over
  * several CTAs, which add their sums with reductions: the summation order is then not fixed (differences ~1e-6); larger
- * launches are deterministic, unless accumulate has KUIPER_GEMM_ANY_ORDER set, which lets them share tiles as well.
+ * launches are deterministic.
  * Any M > 0 is accepted; K % 128 == 0, N % 8 == 0.
  * workspace: kuiper_awq_gemm_workspace_bytes(M, K) bytes (16-byte aligned) for the fp16 copy of x that the kernels read;
  * required.
  * kuiper_awq_gemm_status() synchronously reads the kernels' bounded-wait error words. ---- */
-#define KUIPER_GEMM_ANY_ORDER 2
 KUIPER_API size_t kuiper_awq_gemm_workspace_bytes(int M, int K);
 KUIPER_API int kuiper_awq_gemm_f32(const float* x, const int32_t* qweight, const int32_t* qzeros,
                                    const uint16_t* scales, float* y, const float* residual, int accumulate,
@@ -201,6 +200,13 @@ KUIPER_API int kuiper_awq_gemm_f32(const float* x, const int32_t* qweight, const
 KUIPER_API int kuiper_awq_gemm_f16in_f32(const uint16_t* x16, const int32_t* qweight, const int32_t* qzeros,
                                          const uint16_t* scales, float* y, const float* residual, int accumulate,
                                          int M, int K, int N, int group, kuiper_stream_t stream);
+/* Both calls above for callers that accept any summation order from launches of every size (the engine's accumulating
+ * projections): CTAs may then share the tiles that do not come out evenly.  Exactly one of x (fp32, needs the workspace) and
+ * x16 (fp16) is given, the other is NULL. */
+KUIPER_API int kuiper_awq_gemm_any_order_f32(const float* x, const uint16_t* x16, const int32_t* qweight,
+                                             const int32_t* qzeros, const uint16_t* scales, float* y,
+                                             const float* residual, int accumulate, int M, int K, int N, int group,
+                                             void* workspace, size_t workspace_bytes, kuiper_stream_t stream);
 KUIPER_API int kuiper_awq_gemm_status(void);
 
 /* ---- tensor-parallel exchanges for decode rows over peer-mapped buffers.  No counterpart in the reference (it has no

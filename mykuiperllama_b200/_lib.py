@@ -52,6 +52,7 @@ KERNEL_API = {
     "kuiper_awq_gemm_workspace_bytes": (_sz, [_i32, _i32]),
     "kuiper_awq_gemm_f32": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp, _sz, _vp]),
     "kuiper_awq_gemm_f16in_f32": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp]),
+    "kuiper_awq_gemm_any_order_f32": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp, _sz, _vp]),
     "kuiper_awq_gemm_status": (_i32, []),
     "kuiper_allreduce_buffer_bytes": (_sz, [_i32, _i64]),
     "kuiper_allreduce_state_bytes": (_sz, []),

@@ -190,6 +190,21 @@ def awq_gemm_f16in(x16, qweight, qzeros, scales, y=None, residual=None, accumula
     return y
 
 
+def awq_gemm_any_order(x, qweight, qzeros, scales, y=None, residual=None, accumulate=False, group=128):
+    """awq_gemm (x fp32) or awq_gemm_f16in (x fp16) without a promise about the summation order, whatever the size."""
+    _dev(x, qweight, qzeros, scales)
+    M, K = x.shape
+    N = qweight.shape[1] * 8
+    if y is None:
+        y = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    half = x.dtype == torch.float16
+    workspace = None if half else awq_gemm_workspace(M, K, x.device)
+    check(kernels().kuiper_awq_gemm_any_order_f32(None if half else _ptr(x), _ptr(x) if half else None, _ptr(qweight), _ptr(qzeros),
+                                                  _ptr(scales), _ptr(y), _ptr(residual), int(bool(accumulate)), M, K, N, group,
+                                                  _ptr(workspace), 0 if half else workspace.numel(), _stream()))
+    return y
+
+
 def awq_gemm_status() -> None:
     check(kernels().kuiper_awq_gemm_status())
 

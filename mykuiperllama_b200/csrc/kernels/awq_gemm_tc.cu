@@ -1068,12 +1068,10 @@ extern "C" size_t kuiper_awq_gemm_workspace_bytes(int M, int K) {
     return (size_t(M) * size_t(K) * sizeof(__half) + 255) / 256 * 256;  // fp16 copy of the activations
 }
 
-// Shared by the two entry points: x is fp32 (converted into the workspace first) or already fp16 (x16, no workspace).
+// Shared by the entry points: x is fp32 (converted into the workspace first) or already fp16 (x16, no workspace).
 static int gemm_common(const float* x, const __half* x16_in, const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales,
-                       float* y, const float* residual, int accumulate, int M, int K, int N, int group, void* workspace,
-                       size_t workspace_bytes, kuiper_stream_t stream) {
-    const bool any_order = (accumulate & KUIPER_GEMM_ANY_ORDER) != 0;
-    accumulate &= ~KUIPER_GEMM_ANY_ORDER;
+                       float* y, const float* residual, int accumulate, bool any_order, int M, int K, int N, int group,
+                       void* workspace, size_t workspace_bytes, kuiper_stream_t stream) {
     KUIPER_REQUIRE((x || x16_in) && qweight && qzeros && scales && y, "awq_gemm: null tensor pointer");
     KUIPER_REQUIRE(M > 0 && K > 0 && N > 0, "awq_gemm: empty shape M=%d K=%d N=%d", M, K, N);
     KUIPER_REQUIRE(group == 128, "awq_gemm: group size %d is not supported (128 only)", group);
@@ -1168,13 +1166,21 @@ extern "C" int kuiper_awq_gemm_f32(const float* x, const int32_t* qweight, const
                                    float* y, const float* residual, int accumulate, int M, int K, int N, int group,
                                    void* workspace, size_t workspace_bytes, kuiper_stream_t stream) {
     KUIPER_REQUIRE(x != nullptr, "awq_gemm: null tensor pointer");
-    return gemm_common(x, nullptr, qweight, qzeros, scales, y, residual, accumulate, M, K, N, group, workspace, workspace_bytes, stream);
+    return gemm_common(x, nullptr, qweight, qzeros, scales, y, residual, accumulate, false, M, K, N, group, workspace, workspace_bytes, stream);
 }
 
 extern "C" int kuiper_awq_gemm_f16in_f32(const uint16_t* x16, const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales,
                                          float* y, const float* residual, int accumulate, int M, int K, int N, int group,
                                          kuiper_stream_t stream) {
     KUIPER_REQUIRE(x16 != nullptr, "awq_gemm_f16in: null tensor pointer");
-    return gemm_common(nullptr, reinterpret_cast<const __half*>(x16), qweight, qzeros, scales, y, residual, accumulate, M, K, N, group,
+    return gemm_common(nullptr, reinterpret_cast<const __half*>(x16), qweight, qzeros, scales, y, residual, accumulate, false, M, K, N, group,
                        nullptr, 0, stream);
+}
+
+extern "C" int kuiper_awq_gemm_any_order_f32(const float* x, const uint16_t* x16, const int32_t* qweight, const int32_t* qzeros,
+                                             const uint16_t* scales, float* y, const float* residual, int accumulate, int M, int K, int N,
+                                             int group, void* workspace, size_t workspace_bytes, kuiper_stream_t stream) {
+    KUIPER_REQUIRE((x != nullptr) != (x16 != nullptr), "awq_gemm_any_order: exactly one of x and x16 is given");
+    return gemm_common(x, reinterpret_cast<const __half*>(x16), qweight, qzeros, scales, y, residual, accumulate, true, M, K, N, group,
+                       workspace, workspace_bytes, stream);
 }

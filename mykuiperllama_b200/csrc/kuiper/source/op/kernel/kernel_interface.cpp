@@ -122,16 +122,17 @@ void matmul_kernel_quant_gemm_cu(const Tensor& input, const Tensor& qweight, con
     const int32_t M = int32_t(input.size() / size_t(K));
     CHECK_EQ(output.size(), size_t(M) * size_t(N));
     if (input.data_type() == base::DataType::DataTypeFp16) {  // normalised / activated rows that already are fp16
-        KERNEL_OK(kuiper_awq_gemm_f16in_f32(input.ptr<uint16_t>(), qweight.ptr<int32_t>(), qzeros.ptr<int32_t>(),
-                                            scales.ptr<uint16_t>(), out_ptr<float>(output),
-                                            residual ? residual->ptr<float>() : nullptr, (accumulate ? 1 : 0) | KUIPER_GEMM_ANY_ORDER, M,
-                                            K, N, group_size, as_stream(stream)));
+        KERNEL_OK(kuiper_awq_gemm_any_order_f32(nullptr, input.ptr<uint16_t>(), qweight.ptr<int32_t>(), qzeros.ptr<int32_t>(),
+                                                scales.ptr<uint16_t>(), out_ptr<float>(output),
+                                                residual ? residual->ptr<float>() : nullptr, accumulate ? 1 : 0, M, K, N, group_size,
+                                                nullptr, 0, as_stream(stream)));
         return;
     }
-    KERNEL_OK(kuiper_awq_gemm_f32(input.ptr<float>(), qweight.ptr<int32_t>(), qzeros.ptr<int32_t>(), scales.ptr<uint16_t>(),
-                                  out_ptr<float>(output), residual ? residual->ptr<float>() : nullptr, (accumulate ? 1 : 0) | KUIPER_GEMM_ANY_ORDER, M,
-                                  K, N, group_size, workspace.is_empty() ? nullptr : out_ptr<void>(workspace),
-                                  workspace.is_empty() ? 0 : workspace.byte_size(), as_stream(stream)));
+    KERNEL_OK(kuiper_awq_gemm_any_order_f32(input.ptr<float>(), nullptr, qweight.ptr<int32_t>(), qzeros.ptr<int32_t>(),
+                                            scales.ptr<uint16_t>(), out_ptr<float>(output), residual ? residual->ptr<float>() : nullptr,
+                                            accumulate ? 1 : 0, M, K, N, group_size,
+                                            workspace.is_empty() ? nullptr : out_ptr<void>(workspace),
+                                            workspace.is_empty() ? 0 : workspace.byte_size(), as_stream(stream)));
 }
 
 void rmsnorm_kernel_cu(const Tensor& input, const Tensor& weight, const Tensor& output, float eps, void* stream) {
