@@ -119,8 +119,9 @@ private:
     bool rows_are_chunk_ = false;
     int32_t chunk_pos0_ = 0, chunk_slot_ = 0;
     static constexpr int32_t kPrefillAttentionMinRows = 16;
-    // from here on the GEMM's tiles are mostly whole ones that it stores without adding (fewer rows: every tile is shared by
-    // several CTAs, and zeroing it in the rotary kernel costs nothing extra)
+    // from here on the column projections overwrite their outputs: gate|up, the widest buffer, then has mostly whole tiles
+    // that the GEMM stores without adding (with fewer rows every tile is shared by several CTAs, and zeroing it in the rotary
+    // kernel costs nothing extra); q|k|v, a quarter of it, is zeroed by the GEMM call until it has whole tiles too
     static constexpr int32_t kOverwriteRows = 512;
 };
 

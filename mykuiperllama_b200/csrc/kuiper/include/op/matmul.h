@@ -51,8 +51,10 @@ public:
     // the addition cost a 2048-row chunk of the Qwen3-8B shape 150 us a layer.
     void set_overwrite_rows(int32_t rows) { overwrite_rows_ = rows; }
     bool overwrites(int32_t rows) const {
-        return is_quant_layer_ && act_mode_ != 0 && overwrite_rows_ > 0 && rows >= overwrite_rows_ && gemm_min_rows_ > 0 && rows >= gemm_min_rows_;
+        return is_quant_layer_ && act_mode_ != 0 && overwrite_rows_ > 0 && gemm_min_rows_ > 0 && rows >= overwrite_from();
     }
+    // fewest rows of a pass that overwrites (where passes do): the GEMV, which serves what the GEMM entry does not, only adds
+    int32_t overwrite_from() const { return overwrite_rows_ > gemm_min_rows_ ? overwrite_rows_ : gemm_min_rows_; }
     // scratch of the split-K kernel: kernel::matmul_quant_workspace_bytes(M, K, N) bytes, zero-initialised once
     void set_workspace(const tensor::Tensor& workspace);
     // scratch of the tensor-core path: kernel::matmul_quant_gemm_workspace_bytes(max rows, dim1) bytes, no

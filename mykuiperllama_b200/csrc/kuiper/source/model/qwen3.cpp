@@ -614,50 +614,56 @@ base::Status Qwen3Model::run_pass(int32_t M, bool inputs_settled) {
     RETURN_IF_ERROR(embedding_->forward(tokens, h));
     // a prompt chunk writes the projections' outputs anew in every layer; decode passes add into zeroed ones
     const bool overwrite = !layers_.empty() && layers_[0].qkv->overwrites(M);
-    for (Qwen3Layer& L : layers_) {
-        L.rope->set_clear_enabled(!overwrite);
-        if (accumulate_cols_) {
-            RETURN_IF_ERROR(L.qkv->forward(h, qkv));  // RMSNorm fused into the projection
-        } else {
-            RETURN_IF_ERROR(L.input_norm->forward(h, xn));
-            RETURN_IF_ERROR(L.qkv->forward(xn, qkv));
-        }
-        if (accumulate_cols_ && inputs_settled && slots_distinct_) {
-            // decode batch: rotary, KV append and attention in one kernel; every cache row but the one appended
-            // here is older than this pass
-            RETURN_IF_ERROR(L.rope->forward_with_attention(qkv, pos, slot, cos_t, sin_t, seq_len, att, 1));
-        } else {
-            RETURN_IF_ERROR(L.rope->forward(qkv, pos, slot, cos_t, sin_t, q));
-            // the rotary kernel just before appended one cache row per token row of this pass; when the rows of a
-            // sequence lie within M consecutive positions, every cache row below seq_len - M is older than this pass.
-            // The promise also covers seq_len / slot, so it is only made when those were settled before the pass
-            // (kernels under programmatic dependent launch may start ahead of earlier copies of the same pass).
-            if (rows_are_chunk_ && !inputs_settled) {
-                // prompt chunk of one sequence: tiled causal attention, K / V tiles shared by a block of query rows
-                RETURN_IF_ERROR(L.mha->forward_prefill(q, chunk_pos0_, chunk_slot_, att));
+    auto run_layers = [&]() -> base::Status {
+        for (Qwen3Layer& L : layers_) {
+            L.rope->set_clear_enabled(!overwrite);
+            if (accumulate_cols_) {
+                RETURN_IF_ERROR(L.qkv->forward(h, qkv));  // RMSNorm fused into the projection
             } else {
-                L.mha->set_fresh_rows(rows_compact_ && inputs_settled ? M : -1);
-                RETURN_IF_ERROR(L.mha->forward(q, seq_len, slot, att));
+                RETURN_IF_ERROR(L.input_norm->forward(h, xn));
+                RETURN_IF_ERROR(L.qkv->forward(xn, qkv));
+            }
+            if (accumulate_cols_ && inputs_settled && slots_distinct_) {
+                // decode batch: rotary, KV append and attention in one kernel; every cache row but the one appended
+                // here is older than this pass
+                RETURN_IF_ERROR(L.rope->forward_with_attention(qkv, pos, slot, cos_t, sin_t, seq_len, att, 1));
+            } else {
+                RETURN_IF_ERROR(L.rope->forward(qkv, pos, slot, cos_t, sin_t, q));
+                // the rotary kernel just before appended one cache row per token row of this pass; when the rows of a
+                // sequence lie within M consecutive positions, every cache row below seq_len - M is older than this pass.
+                // The promise also covers seq_len / slot, so it is only made when those were settled before the pass
+                // (kernels under programmatic dependent launch may start ahead of earlier copies of the same pass).
+                if (rows_are_chunk_ && !inputs_settled) {
+                    // prompt chunk of one sequence: tiled causal attention, K / V tiles shared by a block of query rows
+                    RETURN_IF_ERROR(L.mha->forward_prefill(q, chunk_pos0_, chunk_slot_, att));
+                } else {
+                    L.mha->set_fresh_rows(rows_compact_ && inputs_settled ? M : -1);
+                    RETURN_IF_ERROR(L.mha->forward(q, seq_len, slot, att));
+                }
+            }
+            RETURN_IF_ERROR(project_and_reduce(*L.o, att));
+            if (accumulate_cols_) {
+                RETURN_IF_ERROR(L.gate_up->forward(h, gu));
+            } else {
+                RETURN_IF_ERROR(L.post_norm->forward(h, xn2));
+                RETURN_IF_ERROR(L.gate_up->forward(xn2, gu));
+            }
+            if (accumulate_) {
+                RETURN_IF_ERROR(project_and_reduce(*L.down, gu));  // SwiGLU fused into the projection
+            } else {
+                RETURN_IF_ERROR(L.swiglu->forward(gu, act));
+                RETURN_IF_ERROR(project_and_reduce(*L.down, act));
             }
         }
-        RETURN_IF_ERROR(project_and_reduce(*L.o, att));
-        if (accumulate_cols_) {
-            RETURN_IF_ERROR(L.gate_up->forward(h, gu));
-        } else {
-            RETURN_IF_ERROR(L.post_norm->forward(h, xn2));
-            RETURN_IF_ERROR(L.gate_up->forward(xn2, gu));
-        }
-        if (accumulate_) {
-            RETURN_IF_ERROR(project_and_reduce(*L.down, gu));  // SwiGLU fused into the projection
-        } else {
-            RETURN_IF_ERROR(L.swiglu->forward(gu, act));
-            RETURN_IF_ERROR(project_and_reduce(*L.down, act));
-        }
-    }
-    // the next pass that adds finds zeros again: it has fewer than kOverwriteRows rows (the rotary kernel of its first layer
-    // zeroes gate|up)
+        return base::error::success();
+    };
+    const base::Status layers_done = run_layers();
+    // the next pass that adds finds zeros again, after a layer that failed as well: it has fewer rows than the smallest pass that
+    // overwrites (the rotary kernel of its first layer zeroes gate|up)
     if (overwrite)
-        CUDA_OK(cudaMemsetAsync(const_cast<float*>(qkv.ptr<float>()), 0, size_t(kOverwriteRows) * QKV * sizeof(float), stream()));
+        CUDA_OK(cudaMemsetAsync(const_cast<float*>(qkv.ptr<float>()), 0, size_t(layers_[0].qkv->overwrite_from()) * QKV * sizeof(float),
+                                stream()));
+    if (!layers_done) return layers_done;
     if (logit_rows_ > 0) {
         // logits only for the last logit_rows_ rows of the pass
         const int32_t r0 = M - logit_rows_;
