@@ -41,20 +41,26 @@ public:
     // no fused prologue ([max rows, dim1] fp32)
     void set_norm_scratch(const tensor::Tensor& scratch) { norm_scratch_ = scratch; }
     // quantised layers, fp16-operand mode: inputs of at least this many rows go to the GEMM entry (packed-word kernel up to
-    // 32 rows, tcgen05 tiles beyond) instead of the GEMV in passes of four rows (0 = never).  One pass of the
-    // GEMV also runs the input norm / SwiGLU itself, which saves four launches a layer: Qwen3-8B decode of two sequences
+    // 32 rows, tcgen05 tiles beyond) instead of the GEMV (0 = never).  Unless this is called the number is 16, and 3 where the
+    // layer loses nothing by it: it accumulates (the GEMM entry adds with reductions, the GEMV of a layer that does not
+    // accumulate sums in a fixed order), the GEMM workspace holds the rows, and N % 32 == 0 (other widths would
+    // round the weight, which the GEMV does not).  Below three rows one pass of the accumulating GEMV, which also runs the input
+    // norm / SwiGLU itself and so saves four launches a layer, is as fast: Qwen3-8B decode of two sequences
     // takes the same time either way (1.82 ms a step, 0.6B 0.71 against 0.82), of three 1.97 against 2.13, of five
     // 2.00 against 3.35.
-    void set_gemm_min_rows(int32_t rows) { gemm_min_rows_ = rows; }
+    void set_gemm_min_rows(int32_t rows) { gemm_min_rows_ = rows < 0 ? 0 : rows; }
     // accumulate mode: passes of at least this many rows overwrite the output instead (0 = never), so that nobody has to
     // zero it; the engine sets it for the projections whose addend is zero.  Clearing gate|up before and reading it back for
     // the addition cost a 2048-row chunk of the Qwen3-8B shape 150 us a layer.
     void set_overwrite_rows(int32_t rows) { overwrite_rows_ = rows; }
     bool overwrites(int32_t rows) const {
-        return is_quant_layer_ && act_mode_ != 0 && overwrite_rows_ > 0 && gemm_min_rows_ > 0 && rows >= overwrite_from();
+        return is_quant_layer_ && act_mode_ != 0 && overwrite_rows_ > 0 && gemm_min_rows_ != 0 && rows >= overwrite_from();
     }
     // fewest rows of a pass that overwrites (where passes do): the GEMV, which serves what the GEMM entry does not, only adds
-    int32_t overwrite_from() const { return overwrite_rows_ > gemm_min_rows_ ? overwrite_rows_ : gemm_min_rows_; }
+    int32_t overwrite_from() const {
+        const int32_t gemm_from = gemm_min_rows_ < 0 ? kGemmRows : gemm_min_rows_;
+        return overwrite_rows_ > gemm_from ? overwrite_rows_ : gemm_from;
+    }
     // scratch of the split-K kernel: kernel::matmul_quant_workspace_bytes(M, K, N) bytes, zero-initialised once
     void set_workspace(const tensor::Tensor& workspace);
     // scratch of the tensor-core path: kernel::matmul_quant_gemm_workspace_bytes(max rows, dim1) bytes, no
@@ -74,6 +80,9 @@ protected:
     base::DataType weight_data_type(int32_t idx) const override;
 
 private:
+    static constexpr int32_t kGemmRows = 16, kGemmRowsAccumulating = 3;
+    bool takes_gemm(int32_t rows) const;
+
     int32_t dim0_ = 0;
     int32_t dim1_ = 0;
     bool has_residual_ = false;
@@ -86,7 +95,7 @@ private:
     tensor::Tensor gemm_workspace_;
     tensor::Tensor norm_scratch_;
     tensor::Tensor tickets_;
-    int32_t gemm_min_rows_ = 3;
+    int32_t gemm_min_rows_ = -1;  // -1: the layer's own rule
     int32_t overwrite_rows_ = 0;
 };
 }  // namespace op

@@ -12,7 +12,7 @@ MatmulLayer::MatmulLayer(base::DeviceType device_type, int32_t dim0, int32_t dim
     reset_output_size(1);
     reset_weights_size(is_quant_layer ? 2 : 1);
     if (is_quant_layer) group_size_ = 128;
-    if (const char* env = std::getenv("KUIPER_GEMM_MIN_ROWS")) gemm_min_rows_ = std::atoi(env);  // measurement aid
+    if (const char* env = std::getenv("KUIPER_GEMM_MIN_ROWS")) set_gemm_min_rows(std::atoi(env));  // measurement aid
 }
 
 base::DataType MatmulLayer::weight_data_type(int32_t) const {
@@ -66,6 +66,14 @@ base::Status MatmulLayer::check() const {
     return base::error::success();
 }
 
+bool MatmulLayer::takes_gemm(int32_t rows) const {
+    if (!is_quant_layer_ || act_mode_ == 0) return false;
+    if (gemm_min_rows_ >= 0) return gemm_min_rows_ > 0 && rows >= gemm_min_rows_;
+    if (rows >= kGemmRows) return true;
+    return rows >= kGemmRowsAccumulating && accumulate_ && dim0_ % 32 == 0 && !gemm_workspace_.is_empty() &&
+           gemm_workspace_.byte_size() >= kernel::matmul_quant_gemm_workspace_bytes(rows, dim1_);
+}
+
 base::Status MatmulLayer::forward() {
     base::Status status = check();
     if (!status) return status;
@@ -73,7 +81,7 @@ base::Status MatmulLayer::forward() {
     const int32_t M = int32_t(get_input(0).size() / (size_t(dim1_) * (input_swiglu_ ? 2 : 1)));
     if (input_swiglu_ && !(is_quant_layer_ && accumulate_ && input_norm_.is_empty()))
         return base::error::invalid_argument("the fused SwiGLU input needs a quantised layer in accumulate mode without a norm");
-    if (is_quant_layer_ && act_mode_ != 0 && gemm_min_rows_ > 0 && M >= gemm_min_rows_) {
+    if (takes_gemm(M)) {
         // enough rows for the tensor cores: x and the dequantised weight go through tcgen05 as fp16
         if (accumulate_ && has_residual_) return base::error::invalid_argument("accumulate mode takes no residual input");
         const tensor::Tensor* x = &get_input(0);

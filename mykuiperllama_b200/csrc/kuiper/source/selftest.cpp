@@ -7,6 +7,8 @@
 // to_cpu / to_cuda, borrowed pointers, assgin) and the add operator through the kernel
 // registry (test/test_op/test_op_add.cpp:7-91) plus the VecAddLayer the reference never
 // exercises.  gtest is not a dependency here: each EXPECT appends a line to the report.
+#include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <numeric>
 #include <sstream>
@@ -213,6 +215,100 @@ void test_cuda(Report& rep) {
     }
 }
 
+// a quantised projection with its operands on both sides: random packed words, scales of about 2^-7, inputs in [-1, 1)
+struct QuantCase {
+    int32_t M, K, N;
+    std::vector<uint32_t> qw, qz;
+    std::vector<uint16_t> scales;
+    std::vector<float> x;
+    Tensor tx, ty;
+    op::MatmulLayer layer;
+    std::shared_ptr<kernel::CudaConfig> cfg = std::make_shared<kernel::CudaConfig>();
+
+    template <typename T>
+    static Tensor upload(DataType type, std::vector<int32_t> dims, const std::vector<T>& v) {
+        Tensor t(type, std::move(dims), true, base::CUDADeviceAllocatorFactory::get_instance());
+        cudaMemcpy(t.ptr<void>(), v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+        return t;
+    }
+    QuantCase(Report& rep, int32_t m, int32_t k, int32_t n)
+        : M(m), K(k), N(n), qw(size_t(k) * n / 8), qz(size_t(k) / 128 * n / 8), scales(size_t(k) / 128 * n), x(size_t(m) * k),
+          layer(DeviceType::DeviceCUDA, n, k, true) {
+        uint32_t state = 12345u + uint32_t(m * 7 + k + n);
+        auto next = [&] { return (state = state * 1664525u + 1013904223u) >> 8; };  // 24 random bits
+        for (uint32_t& w : qw) w = next() ^ (next() << 16);
+        for (uint32_t& w : qz) w = next() ^ (next() << 16);
+        for (uint16_t& s : scales) s = uint16_t((8u << 10) | (next() & 1023u));
+        for (float& v : x) v = float(next()) / 8388608.f - 1.f;
+        cfg->create();
+        layer.set_cuda_config(cfg);
+        EXPECT(bool(layer.set_weight(0, upload(DataType::DataTypeInt32, {K, N / 8}, qw))));
+        EXPECT(bool(layer.set_weight(1, upload(DataType::DataTypeInt32, {K / 128, N / 8}, qz))));
+        layer.set_scales(upload(DataType::DataTypeFp16, {K / 128, N}, scales));
+        layer.set_workspace(scratch(kernel::matmul_quant_workspace_bytes(M, K, N)));
+        tx = upload(DataType::DataTypeFp32, {M, K}, x);
+        ty = Tensor(DataType::DataTypeFp32, std::vector<int32_t>{M, N}, true, base::CUDADeviceAllocatorFactory::get_instance());
+    }
+    static Tensor scratch(size_t bytes) {
+        Tensor t(DataType::DataTypeFp32, int32_t(bytes / 4 + 1), true, base::CUDADeviceAllocatorFactory::get_instance());
+        cudaMemset(t.ptr<void>(), 0, t.byte_size());
+        return t;
+    }
+    std::vector<float> run(Report& rep) {
+        cudaMemset(ty.ptr<void>(), 0, ty.byte_size());
+        cudaDeviceSynchronize();
+        EXPECT(bool(layer.forward(tx, ty)));
+        cudaStreamSynchronize(cfg->stream());
+        std::vector<float> y(ty.size());
+        cudaMemcpy(y.data(), ty.ptr<void>(), ty.byte_size(), cudaMemcpyDeviceToHost);
+        return y;
+    }
+    // largest |y - x . W| over the largest |x . W|, in 64 bits
+    double error(const std::vector<float>& y) const {
+        static const int place[8] = {0, 4, 1, 5, 2, 6, 3, 7};  // nibble of logical column c
+        double worst = 0, top = 0;
+        std::vector<double> w(size_t(K), 0.0);
+        for (int32_t n = 0; n < N; n++) {
+            for (int32_t k = 0; k < K; k++) {
+                const size_t word = size_t(n) / 8, shift = size_t(4 * place[n % 8]), g = size_t(k) / 128;
+                const int q = int(qw[size_t(k) * (N / 8) + word] >> shift) & 15, z = int(qz[g * (N / 8) + word] >> shift) & 15;
+                w[size_t(k)] = (q - z) * (1.0 + (scales[g * N + size_t(n)] & 1023) / 1024.0) / 128.0;
+            }
+            for (int32_t m = 0; m < M; m++) {
+                double sum = 0;
+                for (int32_t k = 0; k < K; k++) sum += double(x[size_t(m) * K + size_t(k)]) * w[size_t(k)];
+                worst = std::max(worst, std::abs(sum - double(y[size_t(m) * N + size_t(n)])));
+                top = std::max(top, std::abs(sum));
+            }
+        }
+        return worst / top;
+    }
+};
+
+// a few rows through a layer that has not asked for any summation order: what the GEMV gives
+void test_matmul_rows_cuda(Report& rep) {
+    const double half = 1e-3;  // x rounded to fp16, 2^-12 per product on average
+    {  // the GEMV's workspace alone
+        QuantCase c(rep, 8, 256, 128);
+        EXPECT(c.error(c.run(rep)) <= half);
+        c.layer.set_accumulate(true);  // onto zeros
+        EXPECT(c.error(c.run(rep)) <= half);
+    }
+    {  // a width the GEMV multiplies in fp32, weights as they are: K fp32 roundings
+        QuantCase c(rep, 8, 256, 136);
+        c.layer.set_gemm_workspace(QuantCase::scratch(kernel::matmul_quant_gemm_workspace_bytes(c.M, c.K)));
+        EXPECT(c.error(c.run(rep)) <= 256 * 0x1p-24);
+    }
+    for (bool accumulate : {false, true}) {  // K in 32 groups: a sum of many partial sums
+        QuantCase c(rep, 8, 4096, 512);
+        c.layer.set_gemm_workspace(QuantCase::scratch(kernel::matmul_quant_gemm_workspace_bytes(c.M, c.K)));
+        c.layer.set_accumulate(accumulate);
+        const std::vector<float> first = c.run(rep);
+        EXPECT(c.error(first) <= half);
+        for (int i = 0; i < 10 && !accumulate; i++) EXPECT(c.run(rep) == first);  // the order is fixed
+    }
+}
+
 }  // namespace
 
 extern "C" int kuiper_selftest(int use_cuda, char* report, size_t report_bytes) {
@@ -221,7 +317,10 @@ extern "C" int kuiper_selftest(int use_cuda, char* report, size_t report_bytes) 
     test_buffer_cpu(rep);
     test_tensor_cpu(rep);
     test_layer_cpu(rep);
-    if (use_cuda) test_cuda(rep);
+    if (use_cuda) {
+        test_cuda(rep);
+        test_matmul_rows_cuda(rep);
+    }
     rep.out << rep.passed << " checks passed, " << rep.failed << " failed\n";
     if (report && report_bytes > 0) {
         const std::string s = rep.out.str();
