@@ -108,7 +108,7 @@ void matmul_kernel_quant_accum_cu(const Tensor& input, const Tensor& qweight, co
 }
 
 void matmul_kernel_quant_gemm_cu(const Tensor& input, const Tensor& qweight, const Tensor& qzeros, const Tensor& scales,
-                                 const Tensor& output, const Tensor* residual, bool accumulate, int32_t group_size,
+                                 const Tensor& output, const Tensor* residual, bool accumulate, bool any_order, int32_t group_size,
                                  const Tensor& workspace, void* stream) {
     require_cuda(input, "matmul input");
     require_cuda(qweight, "matmul qweight");
@@ -121,18 +121,22 @@ void matmul_kernel_quant_gemm_cu(const Tensor& input, const Tensor& qweight, con
     CHECK_EQ(input.size() % size_t(K), size_t(0));
     const int32_t M = int32_t(input.size() / size_t(K));
     CHECK_EQ(output.size(), size_t(M) * size_t(N));
-    if (input.data_type() == base::DataType::DataTypeFp16) {  // normalised / activated rows that already are fp16
-        KERNEL_OK(kuiper_awq_gemm_any_order_f32(nullptr, input.ptr<uint16_t>(), qweight.ptr<int32_t>(), qzeros.ptr<int32_t>(),
-                                                scales.ptr<uint16_t>(), out_ptr<float>(output),
-                                                residual ? residual->ptr<float>() : nullptr, accumulate ? 1 : 0, M, K, N, group_size,
-                                                nullptr, 0, as_stream(stream)));
-        return;
-    }
-    KERNEL_OK(kuiper_awq_gemm_any_order_f32(input.ptr<float>(), nullptr, qweight.ptr<int32_t>(), qzeros.ptr<int32_t>(),
-                                            scales.ptr<uint16_t>(), out_ptr<float>(output), residual ? residual->ptr<float>() : nullptr,
-                                            accumulate ? 1 : 0, M, K, N, group_size,
-                                            workspace.is_empty() ? nullptr : out_ptr<void>(workspace),
-                                            workspace.is_empty() ? 0 : workspace.byte_size(), as_stream(stream)));
+    const bool half = input.data_type() == base::DataType::DataTypeFp16;  // normalised / activated rows that already are fp16
+    const float* x = half ? nullptr : input.ptr<float>();
+    const uint16_t* x16 = half ? input.ptr<uint16_t>() : nullptr;
+    const int32_t *qw = qweight.ptr<int32_t>(), *qz = qzeros.ptr<int32_t>();
+    const uint16_t* s = scales.ptr<uint16_t>();
+    float* y = out_ptr<float>(output);
+    const float* addend = residual ? residual->ptr<float>() : nullptr;
+    void* ws = half || workspace.is_empty() ? nullptr : out_ptr<void>(workspace);
+    const size_t ws_bytes = ws ? workspace.byte_size() : 0;
+    if (any_order)
+        KERNEL_OK(kuiper_awq_gemm_any_order_f32(x, x16, qw, qz, s, y, addend, accumulate ? 1 : 0, M, K, N, group_size, ws, ws_bytes,
+                                                as_stream(stream)));
+    else if (half)
+        KERNEL_OK(kuiper_awq_gemm_f16in_f32(x16, qw, qz, s, y, addend, accumulate ? 1 : 0, M, K, N, group_size, as_stream(stream)));
+    else
+        KERNEL_OK(kuiper_awq_gemm_f32(x, qw, qz, s, y, addend, accumulate ? 1 : 0, M, K, N, group_size, ws, ws_bytes, as_stream(stream)));
 }
 
 void rmsnorm_kernel_cu(const Tensor& input, const Tensor& weight, const Tensor& output, float eps, void* stream) {

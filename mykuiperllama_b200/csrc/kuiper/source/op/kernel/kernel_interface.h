@@ -41,11 +41,12 @@ using MatmulKernelQuantAccum = void (*)(const tensor::Tensor& input, const tenso
                                         const tensor::Tensor* input_norm_weight, float eps, bool input_swiglu,
                                         int32_t act_mode, const tensor::Tensor* tickets, void* stream);
 
-// Path for several rows: output = input . dequant(...) (+ residual), or output += ... when accumulate.
+// Path for several rows: output = input . dequant(...) (+ residual), or output += ... when accumulate.  any_order: large calls may
+// sum in an order that differs from run to run (small ones do, see kuiper_awq_gemm_f32).
 using MatmulKernelQuantGemm = void (*)(const tensor::Tensor& input, const tensor::Tensor& qweight,
                                        const tensor::Tensor& qzeros, const tensor::Tensor& scales,
                                        const tensor::Tensor& output, const tensor::Tensor* residual, bool accumulate,
-                                       int32_t group_size, const tensor::Tensor& workspace, void* stream);
+                                       bool any_order, int32_t group_size, const tensor::Tensor& workspace, void* stream);
 
 using RMSNormKernel = void (*)(const tensor::Tensor& input, const tensor::Tensor& weight, const tensor::Tensor& output,
                                float eps, void* stream);

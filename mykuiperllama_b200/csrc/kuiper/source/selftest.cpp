@@ -307,6 +307,12 @@ void test_matmul_rows_cuda(Report& rep) {
         EXPECT(c.error(first) <= half);
         for (int i = 0; i < 10 && !accumulate; i++) EXPECT(c.run(rep) == first);  // the order is fixed
     }
+    {  // 400 tiles of 128 x 256 rows and columns: large enough for whole tiles, whose order is fixed
+        QuantCase c(rep, 2048, 1024, 6400);
+        c.layer.set_gemm_workspace(QuantCase::scratch(kernel::matmul_quant_gemm_workspace_bytes(c.M, c.K)));
+        const std::vector<float> first = c.run(rep);
+        for (int i = 0; i < 3; i++) EXPECT(c.run(rep) == first);
+    }
 }
 
 }  // namespace
