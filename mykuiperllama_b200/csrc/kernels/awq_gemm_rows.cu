@@ -20,8 +20,8 @@
 // SwiGLU is the operand: two more warps then read them and write the fp16 stage, in turns, which saves a launch of 2 to 3 us
 // before a projection of 4 to 10 us.  A run that leaves a column tile adds its sums to y with
 // reductions, or, where the caller needs a fixed order, writes them to a workspace slot that a second kernel adds up
-// in run order.  More than 32 rows (the ordered form takes any number) run as passes over the same weights (grid.y),
-// which the L2 serves.
+// in run order.  More than 32 rows run as passes over the same weights (grid.y), which the L2 serves; the ordered form takes at
+// most 32 in one launch, so that its slots stay as many whatever the number of rows.
 #include <cuda.h>
 #include <cstring>
 
@@ -379,6 +379,7 @@ struct RowsPlan {
     int nt, passes, occ, tiles, groups, units, run, ctas;
 };
 int g_rows_min_run = 1;  // tuning key "rows_min_run"
+constexpr int kOrderedRows = 32;
 
 RowsPlan plan_rows(int M, int K, int N, bool ordered) {
     RowsPlan r;
@@ -484,14 +485,23 @@ int awq_rows_f32_launch(const float* x, bool swiglu, const int32_t* qweight, con
     return launch_rows_nt<false>(call, plan, swiglu ? kRowsSwiglu : kRowsF32, stream);
 }
 
-// floats of the slots an ordered call writes
+// most rows of awq_rows_ordered_launch
+int awq_rows_ordered_max() { return kOrderedRows; }
+
+// floats of the slots that ordered calls of up to M rows write: the most that any of them needs (two CTAs per SM have fewer
+// slots than three, so 17 rows may need less than 16)
 size_t awq_rows_partial_floats(int M, int K, int N) {
-    const RowsPlan plan = plan_rows(M, K, N, true);
-    return size_t(plan.ctas + plan.tiles) * M * kTileCols;
+    size_t most = 0;
+    for (int m = M < kOrderedRows ? M : kOrderedRows; m > 0; m = m > 16 ? 16 : (m > 8 ? 8 : 0)) {  // the largest call of each plan
+        const RowsPlan plan = plan_rows(m, K, N, true);
+        const size_t floats = size_t(plan.ctas + plan.tiles) * m * kTileCols;
+        if (floats > most) most = floats;
+    }
+    return most;
 }
 
-// y = x . W (+ residual) with a fixed summation order, x as fp16 (x16) or, up to awq_rows_f32_max rows, fp32; partial:
-// awq_rows_partial_floats floats
+// y = x . W (+ residual) with a fixed summation order for up to awq_rows_ordered_max rows, x as fp16 (x16) or, up to
+// awq_rows_f32_max rows, fp32; partial: awq_rows_partial_floats floats
 int awq_rows_ordered_launch(const __half* x16, const float* x32, const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales, float* y,
                             const float* residual, float* partial, int M, int K, int N, cudaStream_t stream) {
     const RowsPlan plan = plan_rows(M, K, N, true);

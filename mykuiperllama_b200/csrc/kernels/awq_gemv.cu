@@ -428,6 +428,7 @@ bool awq_gemv_mma_supported(int K, int N);
 int awq_gemv_mma_status();
 int awq_gemv_mma_max_rows(bool accumulate);
 size_t awq_rows_partial_floats(int M, int K, int N);
+int awq_rows_ordered_max();
 int awq_rows_f32_max();
 int awq_rows_f32_launch(const float* x, bool swiglu, const int32_t* qweight, const int32_t* qzeros, const uint16_t* scales, float* y, int M, int K,
                         int N, cudaStream_t stream);
@@ -448,10 +449,15 @@ int awq_gemv_group_launch(const void* device_table, int n_items, long long units
 using namespace kuiper;
 
 // Workspace of a call of several rows through the packed-word kernel: the counters of the one-row kernels (left alone, they
-// have to stay zero), the slots of the ordered sum, the fp16 activations.
+// have to stay zero), the slots of the ordered sum, the fp16 activations.  Calls of more than awq_rows_ordered_max rows run in
+// blocks of that many that use the same workspace one after another, so it stops growing there; a workspace made for M rows
+// serves every smaller number.
 static size_t gemv_rows_head(int N) { return (size_t((N + 31) / 32 + 1) * sizeof(int) + 255) / 256 * 256; }
 static size_t gemv_rows_x16(int M, int K, int N) { return gemv_rows_head(N) + awq_rows_partial_floats(M, K, N) * sizeof(float); }
-static size_t gemv_rows_workspace_bytes(int M, int K, int N) { return gemv_rows_x16(M, K, N) + size_t(M) * K * sizeof(__half); }
+static size_t gemv_rows_workspace_bytes(int M, int K, int N) {
+    const int block = M < awq_rows_ordered_max() ? M : awq_rows_ordered_max();
+    return gemv_rows_x16(M, K, N) + size_t(block) * K * sizeof(__half);
+}
 
 extern "C" size_t kuiper_awq_gemv_workspace_bytes(int M, int K, int N) {
     if (M <= 0 || K <= 0 || N <= 0) return 0;
@@ -506,13 +512,22 @@ extern "C" int kuiper_awq_gemv_f32(const float* x, const int32_t* qweight, const
         if (mma && M >= g_rows_min && workspace != nullptr && workspace_bytes >= gemv_rows_workspace_bytes(M, K, N) &&
             ((reinterpret_cast<uintptr_t>(workspace) | reinterpret_cast<uintptr_t>(x)) & 15) == 0) {
             __half* x16 = reinterpret_cast<__half*>(static_cast<char*>(workspace) + gemv_rows_x16(M, K, N));
-            const bool direct = M <= awq_rows_f32_max();  // the kernel rounds the rows itself
-            if (!direct) {
-                const int rc = convert_f16_launch(x, x16, int64_t(M) * K / 4, nullptr, 0, st);
+            float* slots = reinterpret_cast<float*>(static_cast<char*>(workspace) + gemv_rows_head(N));
+            // the launches of a block write the rows, the slots and y only after the launch before them, and with it the
+            // last block, has completed
+            for (int m0 = 0; m0 < M; m0 += awq_rows_ordered_max()) {
+                const int rows = M - m0 < awq_rows_ordered_max() ? M - m0 : awq_rows_ordered_max();
+                const bool direct = rows <= awq_rows_f32_max();  // the kernel rounds the rows itself
+                const float* xm = x + size_t(m0) * K;
+                if (!direct) {
+                    const int rc = convert_f16_launch(xm, x16, int64_t(rows) * K / 4, nullptr, 0, st);
+                    if (rc != KUIPER_OK) return rc;
+                }
+                const int rc = awq_rows_ordered_launch(direct ? nullptr : x16, direct ? xm : nullptr, qweight, qzeros, scales, y + size_t(m0) * N,
+                                                       residual ? residual + size_t(m0) * N : nullptr, slots, rows, K, N, st);
                 if (rc != KUIPER_OK) return rc;
             }
-            return awq_rows_ordered_launch(direct ? nullptr : x16, direct ? x : nullptr, qweight, qzeros, scales, y, residual,
-                                           reinterpret_cast<float*>(static_cast<char*>(workspace) + gemv_rows_head(N)), M, K, N, st);
+            return KUIPER_OK;
         }
         KUIPER_REQUIRE(workspace != nullptr && workspace_bytes >= awq_gemv_tma_workspace_bytes(K, N),
                        "awq_gemv: workspace of %zu bytes is too small", workspace_bytes);
