@@ -45,7 +45,7 @@ constexpr int kConsumerWarps = 4;
 constexpr int kThreadsRows = (kConsumerWarps + 1) * 32;
 enum RowsOperand { kRowsF16, kRowsF32, kRowsSwiglu };
 constexpr int rows_threads(int operand) { return kThreadsRows + (operand == kRowsF16 ? 0 : 64); }
-constexpr uint32_t kSpinLimitRows = 1u << 22;
+constexpr int kSpinLimitRows = 1 << 22;  // polls of one wait, about a microsecond each
 
 __device__ int g_rows_wait_error = 0;
 
@@ -62,11 +62,13 @@ struct RowsCall {
     int groups;             // K / 128
     int units;              // column tiles * groups
     int run;                // units per CTA
+    int spins;              // polls after which a wait gives up
+    int drop;               // test aid: this unit of every CTA is never fetched (-1: none)
 };
 
 __device__ __forceinline__ uint32_t rsm(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ bool rows_wait(uint32_t bar, uint32_t parity, bool relaxed) {
-    for (uint32_t spin = 0; spin < kSpinLimitRows; spin++) {
+__device__ __forceinline__ bool rows_wait(uint32_t bar, uint32_t parity, bool relaxed, int spins) {
+    for (int spin = 0; spin < spins; spin++) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -130,7 +132,7 @@ __global__ void __launch_bounds__(rows_threads(OPERAND), OCC) awq_rows_kernel(co
         const int words_per_row = p.N >> 3;
         auto issue_weights = [&](int i, int s) {
             const int u = u0 + i, tile = u / p.groups, group = u - tile * p.groups;
-            if (lane == 0) {
+            if (lane == 0 && i != p.drop) {
                 const int cols = min(kTileCols, p.N - tile * kTileCols);
                 const uint32_t zbytes = uint32_t(cols) >> 1, sbytes = uint32_t(cols) * 2;
                 const uint32_t bar = rsm(&full_bar[s]), w = smem + s * kWeightBytes, aux = aux0 + s * kAux;
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(rows_threads(OPERAND), OCC) awq_rows_kernel(co
         auto issue_x = [&](int i, int s) {
             if constexpr (OPERAND != kRowsF16) return;
             const int u = u0 + i, group = u % p.groups;
-            if (lane < rows)
+            if (lane < rows && i != p.drop)
                 rows_bulk(aux0 + s * kAux + kZeroBytesR + kScaleBytesR + lane * kXPitch,
                           p.x + size_t(m0 + lane) * p.K + group * kGroupRows, kGroupRows * 2, rsm(&full_bar[s]));
             __syncwarp();
@@ -162,17 +164,19 @@ __global__ void __launch_bounds__(rows_threads(OPERAND), OCC) awq_rows_kernel(co
         for (int i = 0; i < ahead; i++) issue_weights(i, i);
         if constexpr (OPERAND == kRowsF16) pdl_wait();
         for (int i = 0; i < ahead; i++) issue_x(i, i);
-        for (int i = ahead; i < n_units; i++) {
-            const int s = i % STAGES;
-            if (!rows_wait(rsm(&empty_bar[s]), uint32_t(i / STAGES - 1) & 1u, true)) {
+        int issued = ahead;
+        for (; issued < n_units; issued++) {
+            const int s = issued % STAGES;
+            if (!rows_wait(rsm(&empty_bar[s]), uint32_t(issued / STAGES - 1) & 1u, true, p.spins)) {
                 if (lane == 0) atomicExch(&g_rows_wait_error, 11);
-                // the copies in flight have to land before the CTA gives its shared memory back
-                for (int j = i - STAGES; j < i; j++) rows_wait(rsm(&full_bar[j % STAGES]), uint32_t(j / STAGES) & 1u, true);
                 break;
             }
-            issue_weights(i, s);
-            issue_x(i, s);
+            issue_weights(issued, s);
+            issue_x(issued, s);
         }
+        // The copies in flight have to land before the CTA gives its shared memory back, whoever's wait ran out: consumers that
+        // gave up no longer wait for them.  Otherwise this costs nothing, the consumers wait for the same copies.
+        for (int j = max(issued - STAGES, 0); j < issued; j++) rows_wait(rsm(&full_bar[j % STAGES]), uint32_t(j / STAGES) & 1u, true, p.spins);
         return;
     }
 
@@ -197,7 +201,7 @@ __global__ void __launch_bounds__(rows_threads(OPERAND), OCC) awq_rows_kernel(co
                 }
                 // a warp sees every other stage of the ring; the wait on the parity is safe because the consumers free the stages
                 // in order and this warp has seen the stage before last filled
-                if (i >= STAGES && !rows_wait(rsm(&empty_bar[s]), uint32_t(i / STAGES - 1) & 1u, true)) {
+                if (i >= STAGES && !rows_wait(rsm(&empty_bar[s]), uint32_t(i / STAGES - 1) & 1u, true, p.spins)) {
                     if (lane == 0) atomicExch(&g_rows_wait_error, 13);
                     return;
                 }
@@ -239,9 +243,9 @@ __global__ void __launch_bounds__(rows_threads(OPERAND), OCC) awq_rows_kernel(co
     bool first_group = group == 0;  // the run holds the first group of the tile it is working on
     for (int i = 0; i < n_units; i++) {
         const int s = i % STAGES;
-        if (!rows_wait(rsm(&full_bar[s]), uint32_t(i / STAGES) & 1u, false)) {
+        if (!rows_wait(rsm(&full_bar[s]), uint32_t(i / STAGES) & 1u, false, p.spins)) {
             if (lane == 0) atomicExch(&g_rows_wait_error, 12);
-            return;  // the producer's own wait runs out later than this one
+            return;  // the producer still waits for the copies in flight
         }
         const uint32_t w = smem + s * kWeightBytes, aux = aux0 + s * kAux;
         float d[4][NT][4], sum[NT][4];
@@ -379,6 +383,7 @@ struct RowsPlan {
     int nt, passes, occ, tiles, groups, units, run, ctas;
 };
 int g_rows_min_run = 1;  // tuning key "rows_min_run"
+int g_rows_spins = kSpinLimitRows, g_rows_drop = -1;  // tuning keys "rows_wait_spins", "rows_drop_unit" (tests of the bounded waits)
 constexpr int kOrderedRows = 32;
 
 RowsPlan plan_rows(int M, int K, int N, bool ordered) {
@@ -441,6 +446,8 @@ bool fill_rows(RowsCall& call, const RowsPlan& plan, const __half* x16, const in
     call.groups = plan.groups;
     call.units = plan.units;
     call.run = plan.run;
+    call.spins = g_rows_spins;
+    call.drop = g_rows_drop;
     return true;
 }
 
@@ -448,6 +455,8 @@ bool fill_rows(RowsCall& call, const RowsPlan& plan, const __half* x16, const in
 
 void awq_rows_set_tuning(const char* key, int value) {
     if (!strcmp(key, "rows_min_run")) g_rows_min_run = value < 1 ? 1 : value;
+    if (!strcmp(key, "rows_wait_spins")) g_rows_spins = value < 1 ? kSpinLimitRows : value;
+    if (!strcmp(key, "rows_drop_unit")) g_rows_drop = value;
 }
 
 int awq_rows_status() {
