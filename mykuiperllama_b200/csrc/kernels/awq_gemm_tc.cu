@@ -34,7 +34,7 @@ namespace {
 constexpr int kBM = 128, kBK = 64;
 constexpr int kGemmThreads = 256;
 constexpr uint32_t kMagicTc = 0x64006400u;
-constexpr uint32_t kSpinLimitTc = 1u << 22;
+constexpr int kSpinLimitTc = 1 << 22;  // polls of one wait, about a microsecond each
 
 __device__ int g_gemm_wait_error = 0;
 
@@ -56,9 +56,9 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) { return uint32_t(_
 __device__ __forceinline__ __half2 tc_u2h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 __device__ __forceinline__ uint32_t tc_h22u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 
-__device__ __forceinline__ bool tc_mbar_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool tc_mbar_wait(uint64_t* bar, uint32_t parity, int spins = kSpinLimitTc) {
     const uint32_t addr = smem_addr(bar);
-    for (uint32_t spin = 0; spin < kSpinLimitTc; spin++) {
+    for (int spin = 0; spin < spins; spin++) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -635,15 +635,16 @@ struct GemmCall4 {
     int whole_tiles;           // tiles that a CTA has to itself; they come first
     int full_units, full_run;  // end of the units of the tile rows of 256 rows; units of them per CTA behind the whole tiles
     int tail_units, tail_run;  // the same for a last tile row of fewer rows
+    int spins;                 // polls after which a wait gives up
+    int drop;                  // test aid: the activations of this stage use of every CTA are never fetched (-1: none)
 };
 
 __global__ void __launch_bounds__(kThreads4, 1) awq_gemm_tc4_kernel(const __grid_constant__ GemmCall4 p) {
     extern __shared__ unsigned char smem_raw[];
     const uint32_t smem = (smem_addr(smem_raw) + 1023u) & ~1023u;
     const uint32_t sA = smem, sB = smem + kStages4 * kStageA4, sY = sB + kStages4 * kStageB4;
-    __shared__ uint64_t full_bar[kStages4], free_bar[kStages4], tile_bar, drained_bar;
+    __shared__ uint64_t full_bar[kStages4], free_bar[kStages4], tile_bar, drained_bar, exit_bar;
     __shared__ uint32_t s_tmem;
-    __shared__ int s_dead;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
     if (tid == 0) {
@@ -654,8 +655,8 @@ __global__ void __launch_bounds__(kThreads4, 1) awq_gemm_tc4_kernel(const __grid
         }
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&drained_bar)), "r"(uint32_t(2 * kHalfThreads4 / 32)));
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&tile_bar)));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&exit_bar)));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        s_dead = 0;
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)), "r"(512u) : "memory");
@@ -712,12 +713,12 @@ __global__ void __launch_bounds__(kThreads4, 1) awq_gemm_tc4_kernel(const __grid
                 const int boxes = p.M - u.mt * kTileM4 > kBM ? 2 : 1;
                 for (int h = 0; h < 2; h++, it++) {
                     const int s = it % kStages4;
-                    if (it >= kStages4 && !tc_mbar_wait(&free_bar[s], uint32_t(it / kStages4 - 1) & 1u)) {
+                    if (it >= kStages4 && !tc_mbar_wait(&free_bar[s], uint32_t(it / kStages4 - 1) & 1u, p.spins)) {
                         atomicExch(&g_gemm_wait_error, 21);
-                        s_dead = 1;
                         dead = true;
                         break;
                     }
+                    if (it == p.drop) continue;
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&full_bar[s])),
                                  "r"(uint32_t(boxes * kStageA2))
                                  : "memory");
@@ -729,9 +730,9 @@ __global__ void __launch_bounds__(kThreads4, 1) awq_gemm_tc4_kernel(const __grid
                             : "memory");
                 }
             }
-            // after a failed wait the copies in flight still have to land before the block may end
-            if (dead)
-                for (int j = it - kStages4 < 0 ? 0 : it - kStages4; j < it; j++) tc_mbar_wait(&full_bar[j % kStages4], uint32_t(j / kStages4) & 1u);
+            // the copies in flight have to land before the block may end, whoever's wait ran out (otherwise this costs nothing)
+            for (int j = it - kStages4 < 0 ? 0 : it - kStages4; j < it; j++)
+                tc_mbar_wait(&full_bar[j % kStages4], uint32_t(j / kStages4) & 1u, p.spins);
         }
     } else if (warp == 16) {
         // ------------------------------------------------------------ MMA issue
@@ -744,16 +745,14 @@ __global__ void __launch_bounds__(kThreads4, 1) awq_gemm_tc4_kernel(const __grid
                 u = i == 0 ? unit_at(0) : unit_after(i - 1, u);
                 const int halves = p.M - u.mt * kTileM4 > kBM ? 2 : 1;
                 // a new tile overwrites the accumulators: every warp has to have read the last one's
-                if (fresh && tiles > 0 && !tc_mbar_wait(&drained_bar, uint32_t(tiles - 1) & 1u)) {
+                if (fresh && tiles > 0 && !tc_mbar_wait(&drained_bar, uint32_t(tiles - 1) & 1u, p.spins)) {
                     atomicExch(&g_gemm_wait_error, 25);
-                    s_dead = 1;
                     break;
                 }
                 for (int h = 0; h < 2; h++, it++) {
                     const int s = it % kStages4;
-                    if (!tc_mbar_wait(&full_bar[s], uint32_t(it / kStages4) & 1u)) {
+                    if (!tc_mbar_wait(&full_bar[s], uint32_t(it / kStages4) & 1u, p.spins)) {
                         atomicExch(&g_gemm_wait_error, 22);
-                        s_dead = 1;
                         dead = true;
                         break;
                     }
@@ -783,6 +782,10 @@ __global__ void __launch_bounds__(kThreads4, 1) awq_gemm_tc4_kernel(const __grid
                                  : "memory");
                 }
             }
+            // every MMA issued is done before the block gives its tensor memory back, whoever's wait ran out (otherwise the
+            // results have waited for them)
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(&exit_bar)) : "memory");
+            tc_mbar_wait(&exit_bar, 0, p.spins);
         }
     } else {
         // ------------------------------------------------------------ dequantisation and results
@@ -810,11 +813,11 @@ __global__ void __launch_bounds__(kThreads4, 1) awq_gemm_tc4_kernel(const __grid
         TileConsts tc;
         auto stage_step = [&](int it, const uint32_t (&w)[8]) {
             const int s = it % kStages4;
-            if (it >= kStages4 && !dead && !tc_mbar_wait(&free_bar[s], uint32_t(it / kStages4 - 1) & 1u)) {
+            if (it >= kStages4 && !dead && !tc_mbar_wait(&free_bar[s], uint32_t(it / kStages4 - 1) & 1u, p.spins)) {
                 atomicExch(&g_gemm_wait_error, 23);
-                s_dead = 1;
                 dead = true;
             }
+            if (dead) return;  // an arrival out of turn could complete a phase that a copy still belongs to
             const uint32_t dst = sB + s * kStageB4;
 #pragma unroll
             for (int r = 0; r < 8; r++) {
@@ -849,9 +852,8 @@ __global__ void __launch_bounds__(kThreads4, 1) awq_gemm_tc4_kernel(const __grid
             if (!tile_ends(i, u.group)) continue;
 
             // ---- results: every MMA of the tile is done (a barrier of its own: a half sees only every other phase of free_bar)
-            if (!dead && !tc_mbar_wait(&tile_bar, uint32_t(tiles++) & 1u)) {
+            if (!dead && !tc_mbar_wait(&tile_bar, uint32_t(tiles++) & 1u, p.spins)) {
                 atomicExch(&g_gemm_wait_error, 24);
-                s_dead = 1;
                 dead = true;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -954,6 +956,7 @@ bool encode_rows_map(CUtensorMap* out, CUtensorMapDataType type, int elem_bytes,
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+int g_gemm_tile_spins = kSpinLimitTc, g_gemm_tile_drop = -1;  // tuning keys "tile_wait_spins", "tile_drop_stage" (tests of the bounded waits)
 int g_gemm_tile_rows = 33;  // tuning key "gemm_tile_rows": fewest rows of a call that takes the 256 x 256 tiles; 0: none
 
 // The 256 x 256 tiles lead everywhere (4096 x 24576: 64 rows 39.7 against 48.6 us, 256 rows 54 / 88, 512 rows 97 / 163, 2048
@@ -990,6 +993,8 @@ int launch_tiles4(const GemmParams& g, const __half* x16, bool share, bool zeroe
     c.m_tiles = (g.M + kTileM4 - 1) / kTileM4;
     c.n_tiles = (g.N + kTileN4 - 1) / kTileN4;
     c.groups = g.K / 128;
+    c.spins = g_gemm_tile_spins;
+    c.drop = g_gemm_tile_drop;
     const int tail = g.M % kTileM4 != 0 ? 1 : 0, ctas = device_sm_count();
     c.full_units = (c.m_tiles - tail) * c.n_tiles * c.groups;
     c.tail_units = tail * c.n_tiles * c.groups;
@@ -1045,6 +1050,8 @@ int convert_f16_launch(const float* x, __half* out, int64_t n4, float* zero, int
 void awq_gemm_set_tuning(const char* key, int value) {
     if (!strcmp(key, "gemm_impl")) g_gemm_impl = value == 3 ? 3 : 2;
     if (!strcmp(key, "gemm_tile_rows")) g_gemm_tile_rows = value < 0 ? 0 : value;
+    if (!strcmp(key, "tile_wait_spins")) g_gemm_tile_spins = value < 1 ? kSpinLimitTc : value;
+    if (!strcmp(key, "tile_drop_stage")) g_gemm_tile_drop = value;
     if (!strcmp(key, "gemm_rows_max")) g_gemm_rows_max = value < 0 ? 0 : value;
     awq_rows_set_tuning(key, value);
     if (!strcmp(key, "gemm_split_k")) g_gemm_split_k = value < 0 ? 0 : value;

@@ -56,3 +56,13 @@ def test_packed_word_projection(M, K, N, call, drop):
             "ordered": "capi.awq_gemv(x, *w)"}[call]
     _process(f"x, w, _ = _case({M}, {K}, {N}, 1)\n"
              f"run(lambda: {call}, kernels().kuiper_awq_gemm_status, 'rows_wait_spins', 'rows_drop_unit', {drop})")
+
+
+# 300 rows: a full tile row and a short one; 2048 x 6144: several tiles of one CTA.  Stage 0 starts a tile, later ones are in the middle
+@pytest.mark.parametrize("M,K,N", [(64, 1024, 2048), (300, 512, 4096), (2048, 512, 6144)])
+@pytest.mark.parametrize("drop", [0, 1, 3, 6])
+def test_tensor_core_tiles(M, K, N, drop):
+    if M < 2048 and drop > 1:
+        pytest.skip("a CTA has one group, which is two stages")
+    _process(f"x, w, _ = _case({M}, {K}, {N}, 1)\n"
+             f"run(lambda: capi.awq_gemm(x, *w), kernels().kuiper_awq_gemm_status, 'tile_wait_spins', 'tile_drop_stage', {drop})")
