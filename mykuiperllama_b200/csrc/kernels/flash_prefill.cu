@@ -268,9 +268,11 @@ int g_prefill_tc_vectors = 1024;
 
 bool flash_prefill_tc_launch(const float* q, const uint16_t* kcache, const uint16_t* vcache, float* out, int M, int Nq, int Nkv, int max_seq,
                              int n_slots, int pos0, int slot, cudaStream_t stream, int* rc);
+void flash_prefill_tc_set_tuning(const char* key, int value);
 
 void flash_prefill_set_tuning(const char* key, int value) {
     if (!strcmp(key, "prefill_tc_vectors")) g_prefill_tc_vectors = value < 0 ? 0 : value;
+    flash_prefill_tc_set_tuning(key, value);
 }
 
 }  // namespace kuiper

@@ -30,7 +30,7 @@ constexpr int kTSlots = 3;
 constexpr int kTQ = 2 * kTSlot;                 // high and low parts of one query tile
 constexpr int kTThreads = 256 + 64;             // two softmax warpgroups, MMA warp, load warp
 constexpr size_t kTSmem = 1024 + 2 * kTQ + kTSlots * kTSlot;
-constexpr uint32_t kTSpin = 1u << 22;
+constexpr int kTSpin = 1 << 22;  // polls of one wait, about a microsecond each
 
 __device__ int g_prefill_wait_error = 0;
 
@@ -40,12 +40,14 @@ struct PrefillTcCall {
     float* out;
     int M, Nq, Nkv, pos0, head0;  // head0: first head of the sequence's slot in the cache
     int R;
+    int spins;  // polls after which a wait gives up
+    int drop;   // test aid: this K or V tile (in the order K0 V0 K1 V1 ...) is never fetched (-1: none)
 };
 
 __device__ __forceinline__ uint32_t ts_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ bool ts_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool ts_wait(uint64_t* bar, uint32_t parity, int spins) {
     const uint32_t addr = ts_u32(bar);
-    for (uint32_t spin = 0; spin < kTSpin; spin++) {
+    for (int spin = 0; spin < spins; spin++) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -104,7 +106,7 @@ __global__ void __launch_bounds__(kTThreads, 1) flash_prefill_tc_kernel(const __
     extern __shared__ unsigned char smem_raw[];
     const uint32_t smem = (ts_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t sQ = smem, sKV = smem + 2 * kTQ;
-    __shared__ uint64_t slot_full[kTSlots], slot_free[kTSlots], s_ready[2], p_ready[2], o_ready[2], q_ready;
+    __shared__ uint64_t slot_full[kTSlots], slot_free[kTSlots], s_ready[2], p_ready[2], o_ready[2], q_ready, exit_bar;
     __shared__ uint32_t s_tmem;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -122,6 +124,7 @@ __global__ void __launch_bounds__(kTThreads, 1) flash_prefill_tc_kernel(const __
             init(&o_ready[w], 1);
         }
         init(&q_ready, 8);
+        init(&exit_bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -145,14 +148,14 @@ __global__ void __launch_bounds__(kTThreads, 1) flash_prefill_tc_kernel(const __
         // ------------------------------------------------------------ K and V tiles
         if (lane == 0) {
             pdl_wait();  // the newest cache rows come from the preceding kernel
-            for (int i = 0; i < 2 * n_tiles; i++) {  // K0 V0 K1 V1 ...
+            int i = 0;
+            for (; i < 2 * n_tiles; i++) {  // K0 V0 K1 V1 ...
                 const int s = i % kTSlots;
-                if (i >= kTSlots && !ts_wait(&slot_free[s], uint32_t(i / kTSlots - 1) & 1u)) {
+                if (i >= kTSlots && !ts_wait(&slot_free[s], uint32_t(i / kTSlots - 1) & 1u, p.spins)) {
                     atomicExch(&g_prefill_wait_error, 31);
-                    // the copies in flight have to land before the block may end
-                    for (int j = i - kTSlots; j < i; j++) ts_wait(&slot_full[j % kTSlots], uint32_t(j / kTSlots) & 1u);
                     break;
                 }
+                if (i == p.drop) continue;
                 const CUtensorMap* map = (i & 1) ? &p.v_map : &p.k_map;
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(ts_u32(&slot_full[s])), "r"(uint32_t(kTSlot)) : "memory");
                 for (int h = 0; h < 2; h++)
@@ -162,6 +165,8 @@ __global__ void __launch_bounds__(kTThreads, 1) flash_prefill_tc_kernel(const __
                         "r"(ts_u32(&slot_full[s]))
                         : "memory");
             }
+            // the copies in flight have to land before the block may end, whoever's wait ran out (otherwise this costs nothing)
+            for (int j = max(i - kTSlots, 0); j < i; j++) ts_wait(&slot_full[j % kTSlots], uint32_t(j / kTSlots) & 1u, p.spins);
         }
     } else if (warp == 8) {
         // ------------------------------------------------------------ MMA issue
@@ -171,7 +176,7 @@ __global__ void __launch_bounds__(kTThreads, 1) flash_prefill_tc_kernel(const __
             const uint32_t idesc_o = idesc_s | (1u << 16);
             bool dead = false;
             auto need = [&](uint64_t* bar, uint32_t parity) {
-                if (dead || ts_wait(bar, parity)) return;
+                if (dead || ts_wait(bar, parity, p.spins)) return;
                 atomicExch(&g_prefill_wait_error, 32);
                 dead = true;
             };
@@ -228,6 +233,9 @@ __global__ void __launch_bounds__(kTThreads, 1) flash_prefill_tc_kernel(const __
                     else
                         scores(w, j + 1);  // its commit also says that O_w is complete up to tile j
                 }
+            // every MMA issued is done before the block gives its tensor memory back, whoever's wait ran out
+            ts_commit(&exit_bar);
+            ts_wait(&exit_bar, 0, p.spins);
         }
     } else {
         // ------------------------------------------------------------ softmax: thread = one query vector
@@ -265,7 +273,7 @@ __global__ void __launch_bounds__(kTThreads, 1) flash_prefill_tc_kernel(const __
         float mx = -INFINITY, sum = 0.f;
         bool dead = false;
         for (int j = 0; j < n_tiles; j++) {
-            if (!ts_wait(&s_ready[w], uint32_t(j) & 1u)) {
+            if (!ts_wait(&s_ready[w], uint32_t(j) & 1u, p.spins)) {
                 atomicExch(&g_prefill_wait_error, 33);
                 dead = true;
                 break;
@@ -326,7 +334,7 @@ __global__ void __launch_bounds__(kTThreads, 1) flash_prefill_tc_kernel(const __
             __syncwarp();
             if (lane == 0) ts_arrive(&p_ready[w]);
         }
-        if (!dead && !ts_wait(&o_ready[w], 0)) {
+        if (!dead && !ts_wait(&o_ready[w], 0, p.spins)) {
             atomicExch(&g_prefill_wait_error, 34);
             dead = true;
         }
@@ -381,6 +389,12 @@ bool encode_cache_map(CUtensorMap* out, const uint16_t* cache, int heads, int ma
 
 }  // namespace
 
+static int g_prefill_spins = kTSpin, g_prefill_drop = -1;  // tuning keys "prefill_wait_spins", "prefill_drop_tile" (tests of the bounded waits)
+void flash_prefill_tc_set_tuning(const char* key, int value) {
+    if (!strcmp(key, "prefill_wait_spins")) g_prefill_spins = value < 1 ? kTSpin : value;
+    if (!strcmp(key, "prefill_drop_tile")) g_prefill_drop = value;
+}
+
 int flash_prefill_tc_status() {
     int v = 0;
     if (cudaMemcpyFromSymbol(&v, g_prefill_wait_error, sizeof(int)) != cudaSuccess) return -1;
@@ -399,6 +413,8 @@ bool flash_prefill_tc_launch(const float* q, const uint16_t* kcache, const uint1
     c.M = M; c.Nq = Nq; c.Nkv = Nkv; c.pos0 = pos0;
     c.head0 = slot * Nkv;
     c.R = Nq / Nkv;
+    c.spins = g_prefill_spins;
+    c.drop = g_prefill_drop;
     static size_t configured[kMaxDevices] = {};
     if (!ensure_dynamic_smem(flash_prefill_tc_kernel, kTSmem, configured)) {
         set_error("flash_prefill: cannot reserve %zu bytes of shared memory", kTSmem);

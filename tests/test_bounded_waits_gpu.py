@@ -66,3 +66,13 @@ def test_tensor_core_tiles(M, K, N, drop):
         pytest.skip("a CTA has one group, which is two stages")
     _process(f"x, w, _ = _case({M}, {K}, {N}, 1)\n"
              f"run(lambda: capi.awq_gemm(x, *w), kernels().kuiper_awq_gemm_status, 'tile_wait_spins', 'tile_drop_stage', {drop})")
+
+
+# tiles alternate K0 V0 K1 V1 ...; 300 rows of 32 / 8 heads are five blocks of one to three tiles
+@pytest.mark.parametrize("drop", [0, 1, 2, 3, 5])
+def test_prefill_attention(drop):
+    _process(f"""
+g = torch.Generator(device="cuda"); g.manual_seed(1)
+q = torch.randn((300, 32, 128), generator=g, device="cuda")
+k, v = (torch.randn((1, 8, 300, 128), generator=g, device="cuda").bfloat16() for _ in range(2))
+run(lambda: capi.flash_prefill(q, k, v, 0, 0), kernels().kuiper_flash_decode_status, 'prefill_wait_spins', 'prefill_drop_tile', {drop})""")
