@@ -291,8 +291,9 @@ KUIPER_API int kuiper_qknorm_rope_kvwrite(float* qkv, const uint16_t* q_norm_w, 
  * ~1e-5; fresh_rows is accepted and ignored), kuiper_set_tuning("flash_mma", 0) selects the SIMT kernel.
  */
 KUIPER_API size_t kuiper_flash_decode_workspace_bytes(int M, int Nq, int D, int max_seq);
-/* health check (synchronises): 5 if the bounded wait of a combining CTA (fused decode kernel) ran out on this device
- * since the last call (the outputs of that launch are zeros) */
+/* health check (synchronises): 5 if a bounded wait ran out on this device since the last call - that of a combining CTA of the
+ * fused decode kernel (the outputs of that launch are zeros) or one of the tensor-core prefill kernel (parts of its output are
+ * not written) - or if the error words cannot be read */
 KUIPER_API int kuiper_flash_decode_status(void);
 KUIPER_API int kuiper_flash_decode(const float* q, const uint16_t* kcache, const uint16_t* vcache,
                         const int32_t* seq_len, const int32_t* slot, float* out,

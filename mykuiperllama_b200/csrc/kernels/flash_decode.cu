@@ -1192,7 +1192,7 @@ size_t flash_slots(int M) {
 }  // namespace
 
 void flash_prefill_set_tuning(const char* key, int value);
-int flash_prefill_tc_status();
+int flash_prefill_tc_status(bool* read);
 
 void flash_decode_set_tuning(const char* key, int value) {
     if (!strcmp(key, "flash_splits")) g_force_splits = value;
@@ -1222,16 +1222,21 @@ extern "C" KUIPER_API int kuiper_flash_trace_read(int64_t* out, int max_values) 
 #endif
 
 extern "C" int kuiper_flash_decode_status(void) {
-    int v = 0;
+    int decode = 0;
     const int zero = 0;
-    if (cudaMemcpyFromSymbol(&v, g_flash_wait_error, sizeof(int)) != cudaSuccess) v = -1;
-    if (v == 0 && flash_prefill_tc_status() != 0) {
-        set_error("flash_prefill: a bounded tensor-core pipeline wait ran out (code %d)", flash_prefill_tc_status());
+    bool read = true;
+    const int prefill = flash_prefill_tc_status(&read);
+    if (!read || cudaMemcpyFromSymbol(&decode, g_flash_wait_error, sizeof(int)) != cudaSuccess) {
+        set_error("flash attention: the error words of the bounded waits cannot be read");
         return KUIPER_INTERNAL_ERROR;
     }
-    if (v == 0) return KUIPER_OK;
-    cudaMemcpyToSymbol(g_flash_wait_error, &zero, sizeof(int));  // reported once
-    set_error("flash_decode: the combining CTA's bounded wait for the other slices ran out (code %d)", v);
+    if (decode != 0) cudaMemcpyToSymbol(g_flash_wait_error, &zero, sizeof(int));  // reported once
+    if (prefill != 0) {
+        set_error("flash_prefill: a bounded tensor-core pipeline wait ran out (code %d)", prefill);
+        return KUIPER_INTERNAL_ERROR;
+    }
+    if (decode == 0) return KUIPER_OK;
+    set_error("flash_decode: the combining CTA's bounded wait for the other slices ran out (code %d)", decode);
     return KUIPER_INTERNAL_ERROR;
 }
 

@@ -395,9 +395,12 @@ void flash_prefill_tc_set_tuning(const char* key, int value) {
     if (!strcmp(key, "prefill_drop_tile")) g_prefill_drop = value;
 }
 
-int flash_prefill_tc_status() {
+// the code of the last wait that ran out, 0 if none did since the last call; *read = false if the word cannot be read
+int flash_prefill_tc_status(bool* read) {
     int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_prefill_wait_error, sizeof(int)) != cudaSuccess) return -1;
+    const int zero = 0;
+    *read = cudaMemcpyFromSymbol(&v, g_prefill_wait_error, sizeof(int)) == cudaSuccess;
+    if (*read && v != 0) cudaMemcpyToSymbol(g_prefill_wait_error, &zero, sizeof(int));  // reported once
     return v;
 }
 

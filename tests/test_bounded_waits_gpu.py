@@ -76,3 +76,12 @@ g = torch.Generator(device="cuda"); g.manual_seed(1)
 q = torch.randn((300, 32, 128), generator=g, device="cuda")
 k, v = (torch.randn((1, 8, 300, 128), generator=g, device="cuda").bfloat16() for _ in range(2))
 run(lambda: capi.flash_prefill(q, k, v, 0, 0), kernels().kuiper_flash_decode_status, 'prefill_wait_spins', 'prefill_drop_tile', {drop})""")
+
+
+def test_prefill_attention_reports_a_wait_once():
+    _process("""
+q = torch.randn((300, 32, 128), device="cuda")
+k, v = (torch.randn((1, 8, 300, 128), device="cuda").bfloat16() for _ in range(2))
+status = kernels().kuiper_flash_decode_status
+run(lambda: capi.flash_prefill(q, k, v, 0, 0), status, 'prefill_wait_spins', 'prefill_drop_tile', 1)
+assert status() == 0  # the launches after the one that failed are in order""")
