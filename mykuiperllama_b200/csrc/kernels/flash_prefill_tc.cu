@@ -294,12 +294,13 @@ __global__ void __launch_bounds__(kTThreads, 1) flash_prefill_tc_kernel(const __
                 t0 = fmaxf(t0, s[c]); t1 = fmaxf(t1, s[c + 1]); t2 = fmaxf(t2, s[c + 2]); t3 = fmaxf(t3, s[c + 3]);
             }
             const float tile_max = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3));
-            // a vector's first tile always holds a visible row (row 0), later ones may hold none (tile_max = -inf)
+            // a vector's first tile always holds a visible row (row 0), later ones may hold none (tile_max = -inf); a visible
+            // score may be -inf too (a product beyond the fp32 range), whose probability is 0
             if (j == 0) {
                 mx = tile_max;
             } else if (__any_sync(0xffffffffu, (tile_max - mx) * kLog2e > 8.f)) {
                 const float next = fmaxf(mx, tile_max);
-                const float corr = exp2f((mx - next) * kLog2e);
+                const float corr = next == -INFINITY ? 1.f : exp2f((mx - next) * kLog2e);
                 mx = next;
                 sum *= corr;
 #pragma unroll 1
@@ -312,7 +313,7 @@ __global__ void __launch_bounds__(kTThreads, 1) flash_prefill_tc_kernel(const __
                     ts_st32(tO + 32 * c, reinterpret_cast<uint32_t*>(o));
                 }
             }
-            const float base = mx * kLog2e;
+            const float base = mx == -INFINITY ? 0.f : mx * kLog2e;
             float a0 = 0.f, a1 = 0.f;
 #pragma unroll
             for (int c = 0; c < 4; c++) {
