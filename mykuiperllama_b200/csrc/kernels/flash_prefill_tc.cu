@@ -12,7 +12,9 @@
 //                     the row sum refer to the same maximum
 //   O_w += P_w . V    A = probability parts in tensor memory (over the scores they came from), B = V tile, MN-major
 // K and V tiles of 128 rows alternate through a ring of three 32 KB slots.  Cache rows past the chunk's end read as zeros
-// (the tensor maps end there), so nothing beyond the written rows is ever multiplied.
+// (the tensor maps end there), so nothing beyond the written rows is ever multiplied.  A hidden row's probability is 0, and 0
+// times a V that is not finite is NaN, so the second product stops at the 16 rows that hold the last one visible to any vector
+// of its query tile (128 / R token rows; the tiled kernel stops at a multiple of 64).
 // Tensor memory: two tiles x (128 columns S / P + 128 columns O) = all 512 columns; one CTA per SM, longest rows first.
 // Every mbarrier wait is bounded; on a timeout an error word is recorded, the block stops and frees its tensor memory.
 #include <cuda.h>
@@ -213,8 +215,10 @@ __global__ void __launch_bounds__(kTThreads, 1) flash_prefill_tc_kernel(const __
                     if (dead) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     // O_w += P_w . V_j; per 32 cache rows: 16 columns of high parts, 16 of low parts
+                    const int seen = p.pos0 + min(vec0 + w * 128 + 127, n_vec - 1) / p.R - j * kTRows;  // last row of the tile that w sees
 #pragma unroll
-                    for (int kk = 0; kk < 8; kk++)
+                    for (int kk = 0; kk < 8; kk++) {
+                        if (kk * 16 > seen) break;
 #pragma unroll
                         for (int part = 0; part < 2; part++) {
                             const uint32_t a = tmem + w * 256 + (kk >> 1) * 32 + part * 16 + (kk & 1) * 8;
@@ -227,6 +231,7 @@ __global__ void __launch_bounds__(kTThreads, 1) flash_prefill_tc_kernel(const __
                                 ::"r"(tmem + w * 256 + 128), "r"(a), "l"(b), "r"(idesc_o), "r"(acc)
                                 : "memory");
                         }
+                    }
                     if (w == 1) ts_commit(&slot_free[s]);
                     if (j + 1 == n_tiles)
                         ts_commit(&o_ready[w]);

@@ -35,3 +35,21 @@ def test_scores_below_the_fp32_range(attend, hidden):
     assert bool((out[:hidden] == 0).all())
     # 16 significant bits of q and of the probabilities (see test_prefill_tc_gpu.py)
     assert float((out[hidden:].double() - ref).abs().max() / ref.abs().max()) <= 5e-5
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("M,pos0,Nq,Nkv,bad", [(300, 0, 32, 8, 100), (300, 0, 16, 8, 100), (300, 0, 64, 8, 191), (300, 128, 32, 8, 228),
+                                               (513, 64, 32, 8, 64 + 127), (256, 0, 32, 8, 255)])
+def test_a_value_row_that_is_not_finite_stays_out_of_earlier_tiles(attend, M, pos0, Nq, Nkv, bad, value):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + bad)
+    q = torch.randn((M, Nq, 128), generator=g, device="cuda")
+    k, v = (torch.randn((1, Nkv, pos0 + M, 128), generator=g, device="cuda").bfloat16() for _ in range(2))
+    clean = attend(q, k, v, pos0, 0)
+    v[:, :, bad] = value
+    out = attend(q, k, v, pos0, 0)
+    first = bad // 64 * 64 - pos0  # earlier rows share no 64-row cache tile with the bad one
+    assert torch.equal(out[:first], clean[:first])
+    assert not bool(torch.isfinite(out[bad - pos0:]).any())
+    ref = _reference(q, k[0], torch.where(torch.isfinite(v[0]), v[0], 0), pos0)[:first]
+    assert float((out[:first].double() - ref).abs().max() / ref.abs().max()) <= 5e-5
