@@ -76,7 +76,7 @@ KUIPER_API int kuiper_awq_dequant_bf16(const int32_t* qweight, const int32_t* qz
  * Scratch for the GEMV: partial sums, fp16 rows and per-tile arrival counters.  The
  * counters must be zero before the first use (kuiper_workspace_init) and are left
  * zero by every call.  Two calls that overlap on the GPU must not share a workspace.
- * A workspace for M rows serves fewer rows too; from 32 rows on its size does not grow.
+ * A workspace for M rows serves fewer rows too; from 128 rows on its size does not grow.
  */
 KUIPER_API size_t kuiper_awq_gemv_workspace_bytes(int M, int K, int N);
 KUIPER_API int kuiper_workspace_init(void* workspace, size_t bytes, kuiper_stream_t stream);

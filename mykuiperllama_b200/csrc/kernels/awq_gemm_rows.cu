@@ -21,7 +21,7 @@
 // before a projection of 4 to 10 us.  A run that leaves a column tile adds its sums to y with
 // reductions, or, where the caller needs a fixed order, writes them to a workspace slot that a second kernel adds up
 // in run order.  More than 32 rows run as passes over the same weights (grid.y), which the L2 serves; the ordered form takes at
-// most 32 in one launch, so that its slots stay as many whatever the number of rows.
+// most 128 in one launch, so that its slots stay as many whatever the number of rows.
 #include <cuda.h>
 #include <cstring>
 
@@ -390,7 +390,8 @@ struct RowsPlan {
 };
 int g_rows_min_run = 1;  // tuning key "rows_min_run"
 int g_rows_rounds = kRoundLimitRows, g_rows_drop = -1;  // tuning keys "rows_wait_spins" (polls), "rows_drop_unit": tests of the bounded waits
-constexpr int kOrderedRows = 32;
+// four passes (51 rows of 3456 x 96, whose launches are what counts: 11.2 us; in blocks of 32 rows 18.8)
+constexpr int kOrderedRows = 128;
 
 RowsPlan plan_rows(int M, int K, int N, bool ordered) {
     RowsPlan r;
@@ -507,7 +508,8 @@ int awq_rows_ordered_max() { return kOrderedRows; }
 // slots than three, so 17 rows may need less than 16)
 size_t awq_rows_partial_floats(int M, int K, int N) {
     size_t most = 0;
-    for (int m = M < kOrderedRows ? M : kOrderedRows; m > 0; m = m > 16 ? 16 : (m > 8 ? 8 : 0)) {  // the largest call of each plan
+    // the largest call of each plan: 8 or 16 rows, or a number of 32-row passes
+    for (int m = M < kOrderedRows ? M : kOrderedRows; m > 0; m = m > 32 ? (m - 1) / 32 * 32 : (m > 16 ? 16 : (m > 8 ? 8 : 0))) {
         const RowsPlan plan = plan_rows(m, K, N, true);
         const size_t floats = size_t(plan.ctas + plan.tiles) * m * kTileCols;
         if (floats > most) most = floats;

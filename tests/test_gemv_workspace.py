@@ -8,18 +8,18 @@ SHAPES = [(9728, 2560), (4096, 24576), (2560, 6144), (128, 32), (2048, 2048), (1
 @pytest.mark.parametrize("K,N", SHAPES)
 def test_size_grows_with_the_rows_and_then_stays(K, N):
     from mykuiperllama_b200._lib import kernels
-    size = [kernels().kuiper_awq_gemv_workspace_bytes(m, K, N) for m in list(range(1, 70)) + [128, 2048, 65536, 1 << 20]]
+    size = [kernels().kuiper_awq_gemv_workspace_bytes(m, K, N) for m in list(range(1, 200)) + [2048, 65536, 1 << 20]]
     assert all(a <= b for a, b in zip(size, size[1:]))
-    assert size[31] == size[-1]
+    assert size[127] == size[-1]
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("M,K,N", [(33, 640, 288), (40, 128, 32), (73, 1152, 1056), (65536 + 40, 128, 32)])
+@pytest.mark.parametrize("M,K,N", [(33, 640, 288), (40, 128, 32), (73, 1152, 1056), (128, 640, 544), (129, 256, 288), (300, 1152, 1056), (65536 + 40, 128, 32)])
 def test_blocks_of_rows_share_a_workspace(cuda, M, K, N):
     import torch
     from test_gemm_rows_gpu import TOL, _case, _err
     x, w, ref = _case(M, K, N, M + K)
-    workspace = cuda.awq_gemv_workspace(32, K, N)
+    workspace = cuda.awq_gemv_workspace(128, K, N)
     res = torch.randn((M, N), device="cuda")
     guard = torch.full((M + 1, N), 7.0, device="cuda")
     cuda.awq_gemv(x, *w, workspace=workspace, out=guard[:M])
