@@ -957,15 +957,45 @@ bool encode_rows_map(CUtensorMap* out, CUtensorMapDataType type, int elem_bytes,
 }
 
 int g_gemm_tile_spins = kSpinLimitTc, g_gemm_tile_drop = -1;  // tuning keys "tile_wait_spins", "tile_drop_stage" (tests of the bounded waits)
+int g_gemm_tile_always = 0;  // tuning key "gemm_tile_always": the tiles also where the other kernel is ahead (tests, measurements)
 int g_gemm_tile_rows = 33;  // tuning key "gemm_tile_rows": fewest rows of a call that takes the 256 x 256 tiles; 0: none
 
-// The 256 x 256 tiles lead everywhere (4096 x 24576: 64 rows 39.7 against 48.6 us, 256 rows 54 / 88, 512 rows 97 / 163, 2048
-// rows 362 / 703) but for one case: between 257 and 511 rows they run a second, short tile row with its own unpacking and
-// results, and the 128-row kernel is ahead where its K split happens to fill one wave of two CTAs per SM (4096 x 6144, 300
-// rows: 34.0 against 38.1 us, 4096 x 2560 23.4 / 28.6; where it does not: 2560 x 6144 39.1 / 24.6).
-bool tiles_pay(int M, int tiles128, int splits128) {
-    const int ctas = tiles128 * splits128, sms = device_sm_count();
-    return M <= 256 || M >= 512 || ctas * 2 < sms * 3 || ctas > 2 * sms;
+// Whether a call takes the 256 x 256 tiles rather than the 128-row kernel.  They lead wherever the latter needs more than one wave of
+// two CTAs per SM or finds nothing to split (4096 x 24576: 64 rows 37 against 45 us, 256 rows 50 / 85, 512 rows 96 / 165, 2048 rows
+// 362 / 703), but for one case: between 257 and 511 rows they run a second, short tile row with its own unpacking and results, and the
+// 128-row kernel is ahead where its K split happens to fill one wave (4096 x 6144, 300 rows: 34.0 against 38.1 us, 4096 x 2560 23.4 /
+// 28.6; where it does not: 2560 x 6144 39.1 / 24.6).
+// Where the split fits one wave, outputs of few tiles leave either kernel a chain of a few stages and a result of 128 or of 256
+// rows to add.  There the estimates below decide; they were fitted to 1146 calls (33 to 2048 rows, K 384 to 9600, N 40 to 24 576) and are 9
+// and 8 % off on average.  Taking the tiles for all of them cost up to 48 % (4096 x 744: 450 rows 17.0 us in the 128-row kernel, 25.1
+// here; 384 x 232: 256 rows 9.1 / 12.4; 1024 x 6144: 700 rows 29.0 / 38.1; the other way round 4096 x 2560, 128 rows: 20.8 / 18.2).  A single
+// group of K and a narrow output (128 x 40: 200 rows 5.7 / 7.1) is the one unsplit call that the 128-row kernel finishes first.
+bool tiles_pay(int M, int K, int N, bool accumulate, int tiles128, int splits128) {
+    const int ctas = tiles128 * splits128, sms = device_sm_count(), groups = K / 128;
+    if (M > 256 && M < 512 && ctas * 2 >= sms * 3 && ctas <= 2 * sms) return false;
+    if (splits128 == 1) return groups > 1 || N > 64 || accumulate;
+    if (ctas > 2 * sms) return true;
+    const float cols = float(N < 256 ? N : 256) / 256.f;
+    // 128-row tiles, us: stages of a CTA (slower once CTAs share SMs), sums added by reductions, one result
+    const float stages = float(2 * groups / splits128);
+    const float rows_us = 2.46f + (ctas * 10 > sms * 7 ? 1.22f : 0.74f) * stages + 0.78f * float(ctas) / float(sms) +
+                          0.96e-6f * float(M) * float(N) * float(splits128) + 3.92f * cols * float(M < 128 ? M : 128) / 128.f;
+    // 256-row tiles, us: the busiest CTA's groups (two MMAs a stage, one in a last tile row of at most 128 rows) and results - a run whose
+    // length does not divide a tile's groups may end in a second tile - and sums added by reductions.  A CTA may have a run of the full
+    // tile rows, one of the last, or both.
+    const int n_tiles = (N + kTileN4 - 1) / kTileN4, last = M % kTileM4;
+    const int full = M / kTileM4 * n_tiles * groups, tail = last ? n_tiles * groups : 0;
+    const int full_run = (full + sms - 1) / sms, tail_run = (tail + sms - 1) / sms;
+    auto run_us = [&](int run, float group_us, float height) {
+        const float results = run == 0 ? 0.f : (run > 1 && groups % run ? 2.f : 1.f);
+        return group_us * float(run) + 5.74f * results * cols * height;
+    };
+    const float full_us = run_us(full_run, 1.77f, 1.f), tail_us = run_us(tail_run, last > 128 ? 1.77f : 1.45f, float(last) / kTileM4);
+    const bool both = (full ? (full + full_run - 1) / full_run : 0) + (tail ? (tail + tail_run - 1) / tail_run : 0) > sms;
+    const float adds = float(N) * 1e-6f * float(groups) *
+                       ((full ? float(M - last) / float(full_run) : 0.f) + (tail ? float(last) / float(tail_run) : 0.f));
+    const float tiles_us = 3.77f + (both ? full_us + tail_us : (full_us > tail_us ? full_us : tail_us)) + 0.31f * adds;
+    return rows_us >= 0.93f * tiles_us;
 }
 
 // zeroes what a launch that overwrites y adds up from several CTAs: columns [col0, N) of every row and the rows from row0 on
@@ -1050,6 +1080,7 @@ int convert_f16_launch(const float* x, __half* out, int64_t n4, float* zero, int
 void awq_gemm_set_tuning(const char* key, int value) {
     if (!strcmp(key, "gemm_impl")) g_gemm_impl = value == 3 ? 3 : 2;
     if (!strcmp(key, "gemm_tile_rows")) g_gemm_tile_rows = value < 0 ? 0 : value;
+    if (!strcmp(key, "gemm_tile_always")) g_gemm_tile_always = value != 0;
     if (!strcmp(key, "tile_wait_spins")) g_gemm_tile_spins = value < 1 ? kSpinLimitTc : value;
     if (!strcmp(key, "tile_drop_stage")) g_gemm_tile_drop = value;
     if (!strcmp(key, "gemm_rows_max")) g_gemm_rows_max = value < 0 ? 0 : value;
@@ -1126,7 +1157,7 @@ static int gemm_common(const float* x, const __half* x16_in, const int32_t* qwei
         if (g_gemm_split_k > 1 && groups % g_gemm_split_k == 0) splits = g_gemm_split_k;  // forced (measurement aid)
     }
     if (g_gemm_impl == 3 && g_gemm_split_k == 1 && g_gemm_tile_rows > 0 && M >= g_gemm_tile_rows && encode_fn_tc() != nullptr &&
-        tiles_pay(M, int(grid2.x * grid2.y), splits)) {
+        (g_gemm_tile_always || tiles_pay(M, K, N, p.mode == 2, int(grid2.x * grid2.y), splits))) {
         const bool share = any_order || splits > 1;
         // where no tile is whole, the launch that converts the activations zeroes y as well
         const bool zero_all = share && n4 > 0 && p.mode != 2 && (M / kTileM4) * ((N + kTileN4 - 1) / kTileN4) < device_sm_count();

@@ -64,7 +64,7 @@ def test_packed_word_projection(M, K, N, call, drop):
 def test_tensor_core_tiles(M, K, N, drop):
     if M < 2048 and drop > 1:
         pytest.skip("a CTA has one group, which is two stages")
-    _process(f"x, w, _ = _case({M}, {K}, {N}, 1)\n"
+    _process(f"capi.set_tuning('gemm_tile_always', 1)\nx, w, _ = _case({M}, {K}, {N}, 1)\n"
              f"run(lambda: capi.awq_gemm(x, *w), kernels().kuiper_awq_gemm_status, 'tile_wait_spins', 'tile_drop_stage', {drop})")
 
 

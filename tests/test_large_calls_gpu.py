@@ -74,7 +74,11 @@ def _all_modes(cuda, calls, M, N, ref):
 def test_whole_and_shared_tiles_of_one_launch(cuda, M, K, N):
     x, w, ref = _case(M, K, N, M + N)
     call = lambda rows, **kw: cuda.awq_gemm_any_order(rows, *w, **kw)
-    _all_modes(cuda, [(call, x), (call, x.half())], M, N, ref)
+    cuda.set_tuning("gemm_tile_always", 1)
+    try:
+        _all_modes(cuda, [(call, x), (call, x.half())], M, N, ref)
+    finally:
+        cuda.set_tuning("gemm_tile_always", 0)
 
 
 # N % 32 != 0 below 33 rows; 257 to 511 rows whose K split fills one wave of two CTAs per SM (3 x 24 tiles, four splits)
