@@ -585,6 +585,12 @@ extern "C" int kuiper_awq_gemv_f32(const float* x, const int32_t* qweight, const
     return KUIPER_OK;
 }
 
+// Three and four gate|up rows fit one pass of the GEMV, whose activation warp reads two rows where the packed-word kernel's two warps
+// hold eight: it is ahead for most of them (us, GEMV / packed words: three rows of 896 x 2560 3.8 / 5.6, 2560 x 24576 12.6 / 15.4;
+// four of 896 x 2560 4.6 / 5.7, 2560 x 6144 6.6 / 7.6), and behind where a long K feeds few columns (three rows of 9728 x 2560 9.9 / 7.9,
+// four 11.0 / 8.1, 12288 x 4096 14.0 / 12.5).
+static bool gate_up_stays(int M, int K, int N) { return (M == 3 && (K < 8192 || K < 3 * N)) || (M == 4 && K < 4096); }
+
 static int awq_gemv_accum_common(const float* x, const uint16_t* norm_w, float eps, bool swiglu, const int32_t* qweight,
                                  const int32_t* qzeros, const uint16_t* scales, float* y, int M, int K, int N, int group,
                                  void* tickets, int act_mode, kuiper_stream_t stream) {
@@ -609,7 +615,7 @@ static int awq_gemv_accum_common(const float* x, const uint16_t* norm_w, float e
     // four 28.2, five rows of 9728 x 2560 5.5 / 13.8).  The engine's decode steps take fp16 rows from a separate launch from
     // three rows on: the wider CTAs of this form leave the next launch less room (Qwen3-8B, five sequences: 51.8 to 53.1 ms
     // against 50.5).
-    if (mma && norm_w == nullptr && M >= 3 && M <= awq_rows_f32_max())
+    if (mma && norm_w == nullptr && M >= 3 && M <= awq_rows_f32_max() && !(swiglu && gate_up_stays(M, K, N)))
         return awq_rows_f32_launch(x, swiglu, qweight, qzeros, scales, y, M, K, N, st);
     const int max_rows = mma ? awq_gemv_mma_max_rows(true) : 2;
     for (int m0 = 0; m0 < M;) {
