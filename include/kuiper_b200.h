@@ -83,8 +83,10 @@ KUIPER_API int kuiper_workspace_init(void* workspace, size_t bytes, kuiper_strea
 
 /*
  * y[M,N] = x[M,K] . dequant(qweight) (+ residual[M,N] if residual != NULL; y may alias
- * residual).  group must be 128, K % 128 == 0, N % 8 == 0.  M <= 8 runs the SIMT
- * dequant-fused GEMV; larger M is processed in row blocks.
+ * residual), summed in a fixed order.  group must be 128, K % 128 == 0, N % 8 == 0.  One row runs the persistent
+ * dequant-fused GEMV, several rows the packed-word kernel in blocks of 128 rows (with a workspace made for fewer rows, or x not
+ * 16-byte aligned: the GEMV, two rows at a time).  KUIPER_ACT_FP32 and N % 32 != 0 (there x stays fp32 in every mode) have
+ * kernels of their own.
  * act_mode: KUIPER_ACT_FP16, KUIPER_ACT_FP32, or KUIPER_ACT_INT16_BLOCK (N % 32 == 0; applies to M == 1, more rows round to fp16).
  */
 KUIPER_API int kuiper_awq_gemv_f32(const float* x, const int32_t* qweight, const int32_t* qzeros,

@@ -1,6 +1,6 @@
 // INT4-AWQ projection of a few token rows (decode batches, short prompts): y[M,N] (+)= x[M,K] . dequant(qweight)[K,N]
-// for two to 32 rows, where the operation should be bound by reading the weights (4096 x 24576: 8 rows 14.7 us, 3.6 TB/s;
-// four-row passes of the GEMV took 28.2, the 128-row tensor-core tiles 45.9).
+// for two to 32 rows, where the operation should be bound by reading the weights (4096 x 24576, ten matrices in turn so that
+// they come from memory: 8 rows 13.8 us, 3.8 TB/s; four-row passes of the GEMV took 27.5, the 128-row tensor-core tiles 45.7).
 // Same placeholder as the GEMV: kuiper/include/op/matmul.h:1-11 of the reference.
 //
 // One packed word costs six integer instructions whatever the number of rows.  Two words of consecutive weight rows
@@ -400,6 +400,7 @@ RowsPlan plan_rows(int M, int K, int N, bool ordered) {
     r.tiles = (N + kTileCols - 1) / kTileCols;
     r.groups = K / kGroupRows;
     r.units = r.tiles * r.groups;
+    // (one matrix over and over, which stays in the L2)
     // Three CTAs per SM stream a large matrix faster (4096 x 24576, 8 rows: 14.8 us against 15.6 with two, 16 rows 17.2 / 19.2).
     // A small one is faster with two, whose runs fill a deeper ring (2560 x 6144, 8 rows: 4.1 us against 4.8, 16 rows 5.7 / 6.2;
     // 9728 x 2560 5.8 / 6.2, 7.9 / 8.4) - but up to eight rows three leave the next launch of a decode step more room (Qwen3-8B,

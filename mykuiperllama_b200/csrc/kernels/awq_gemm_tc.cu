@@ -1053,13 +1053,15 @@ int launch_tiles4(const GemmParams& g, const __half* x16, bool share, bool zeroe
 }
 
 // Calls of up to 32 rows read the weights through the packed-word kernel of awq_gemm_rows.cu, one pass over them: 4096 x 24576
-// 8 rows 14.7, 16 rows 17.2, 32 rows 33.0 us, where the 256 x 256 tiles take 39 us from one row to 64 (they are bound by
-// the dequantisation there) and the 128-row tiles 46.
+// (ten matrices in turn) 8 rows 13.8, 16 rows 16.7, 32 rows 29.6 us, where the 256 x 256 tiles take 38 us from one row to 64 (they
+// are bound by the dequantisation there) and the 128-row tiles 46.
 int g_gemm_rows_max = 32;  // tuning key "gemm_rows_max": most rows of such a call; 0 switches the path off
 
 constexpr int kMaxSplitK = 8;
 int g_gemm_split_k = 1;  // tuning key "gemm_split_k": 0 switches the K split of the third generation off
-int g_gemm_impl = 3;  // 3: mbarrier hand-over to a dedicated MMA warp (default); 2: stages handed over at a block-wide barrier (tuning key "gemm_impl")
+// tuning key "gemm_impl": 3 (as shipped) lets the rules above choose; 2 keeps every call on 128-row tiles handed over at a block-wide
+// barrier (awq_gemm_tc2_kernel)
+int g_gemm_impl = 3;
 
 }  // namespace
 

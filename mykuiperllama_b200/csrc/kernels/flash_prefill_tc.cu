@@ -3,7 +3,9 @@
 // Placeholder it fills: kuiper/include/op/mha.h:1-11 of the reference.
 //
 // The work is a contraction: with q and the probabilities as bf16 high + low parts (16 significant bits, K and V are
-// exact bf16) it takes four products of 128 x 128 x 128 per 128 query vectors and 128 cache rows.  A CTA owns one kv head
+// exact bf16) it takes four products of 128 x 128 x 128 per 128 query vectors and 128 cache rows.  The scheme is the one published
+// for FlashAttention-4: two query tiles in turn, probabilities over their scores in tensor memory, a running maximum that
+// moves only past a factor.  A CTA owns one kv head
 // and 256 query vectors (row, head) = two query tiles of 128; while one tile's softmax runs, the tensor cores work for the
 // other.
 //   S_w = Q_w . K^T   A = q parts in shared memory (K-major, 128-byte swizzle), B = K tile as TMA lays it down
